@@ -111,12 +111,15 @@ typedef struct wfd_problem {
     int32_t ckpt_every;    /* steps between checkpoints; 0 = ceil(sqrt(nt)) */
     int32_t ckpt_format;   /* checkpoint snapshots: WFD_CKPT_FP32, _BF16 or _I16 */
     int32_t lap_store;     /* WFD_LAP_AUTO, _BF16 or _FP32 */
-    int32_t shots_per_cta; /* shots one CTA walks through per step; 0 = automatic */
+    int32_t shots_per_cta; /* shots one CTA of a streaming kernel walks through per step; 0 = automatic
+                              (with tile_rows 0 also the resident kernel, which keeps the
+                              fields of 2D grids up to about 2048^2 on the chip for many
+                              steps, where it is the faster one: the same levels and traces) */
     int32_t group_shots;   /* run the shots in sequential groups of this many, all
                               groups sharing one workspace sized for a group (forward
                               without checkpoints and wfd_misfit_gradient only);
                               0 = all shots at once */
-    int32_t tile_rows;     /* 2D tile height: 16 or 32 rows (0 = 32) */
+    int32_t tile_rows;     /* 2D streaming tile height: 16 or 32 rows (0 = 32, or the resident kernel) */
     int32_t step_block;    /* 2D time steps per kernel launch: 1 or 2 (0 = 1); 2 keeps
                               u_{n+1} in shared memory between the two steps. A forward
                               (no gradient) with the leapfrog update and FP32 fields also
@@ -150,7 +153,9 @@ const char* wfd_last_error(void);
 int wfd_version(void);
 
 /* Workspace size for wfd_forward (with_gradient = 0) or for the
- * forward + backward pair (with_gradient = 1). Host-only, no CUDA call. */
+ * forward + backward pair (with_gradient = 1). Host-only, no CUDA call. It
+ * includes the resident kernel's mailboxes (at most 20 MB) where that kernel may
+ * run; a call whose workspace has no room for them uses the streaming kernels. */
 int wfd_workspace_bytes(const wfd_problem* p, int with_gradient, size_t* bytes);
 
 /*
@@ -190,7 +195,8 @@ int wfd_forward_final(const wfd_problem* p, const float* vel, const float* spong
  * shots; 0 on the fixed ring) and, when grad_wavelet is not NULL,
  * grad_wavelet [nshot][nt][nsrc] = (dF/dwavelet)^T dtraces. Uses the checkpoints
  * of the preceding wfd_forward(save_checkpoints = 1) on the same workspace and
- * inputs, recomputing the forward per segment; one backward per forward.
+ * inputs (give both calls the same workspace_bytes), recomputing the forward
+ * per segment; one backward per forward.
  * Together with wfd_forward this is the reference solver's gradient,
  * cuwave `misfit_gradient(sim, sources, gamma, sensors, observed)` as used by
  * projects/18_fwi/2D_fwi.py:40, for a cotangent the caller chooses.

@@ -180,6 +180,8 @@ struct Geom {
     bool recon;              // the reconstruction adjoint (time reversal, saved frames)
     int band_w, band_cl, band_cr;  // its damped frame: W rows / columns [0, cl), [cr, ld)
     float cs[4], vd_sz;      // staggered first-derivative weights, (dx/dz)^2
+    bool res;                // the resident kernel (fields on the chip), as rf and ra split it
+    ResPlan rf, ra;          // ... forward and recompute; adjoint (gradients only)
 };
 
 // Staggered first-derivative weights of order 2R on a unit grid:
@@ -294,11 +296,44 @@ int check_problem(const wfd_problem* p) {
     return WFD_OK;
 }
 
+// Whether the resident kernel runs the problem, and its splits: the 2D
+// constant-density path with FP32 fields, on grids that fit the chip (for a
+// gradient also with the adjoint's gradient sum in registers), where its estimate
+// is below the streaming kernels' time. Those take about 4 us a step at least and
+// 2 us plus 0.4 M cells per us otherwise (0.44 M for a gradient with two steps per
+// launch, whose recompute overlaps the adjoint). Measured, streaming / resident:
+// forward 256^2 4.1 / 2.2 us, 1024^2 5.7 / 4.1, 2048^2 11.1 / 7.5, 24 shots of
+// 401 x 1203 34 / 22; gradient per step, recompute included, 4 shots of 187 x 243
+// 11.7 / 8.2, 32 shots of 1024^2 with segments of 10 steps 222 / 270 (streamed).
+bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
+    if (p->ndim != 2 || p->field_format != WFD_FIELD_FP32 || p->lap_store != WFD_LAP_AUTO ||
+        p->adjoint_mode != WFD_ADJOINT_CHECKPOINT || p->level_format != WFD_LEVEL_FP32 || p->step_block > 2 ||
+        p->tile_rows > 0 || p->shots_per_cta > 0)  // (a streaming tiling asked for)
+        return false;
+    const double cells = (double)p->nshot * p->nz * p->nx;
+    const double streamed = std::max(4.0, 2.0 + cells / (grad && p->step_block == 2 ? 440e3 : 400e3));
+    const int R = p->order / 2;
+    if (!plan_resident(p->nz, p->nx, R, p->nshot, RES_LEAP, f)) return false;
+    if (!grad) return f->step_us < 0.95 * streamed;
+    if (!plan_resident(p->nz, p->nx, R, p->nshot, RES_ADJOINT, a)) return false;
+    // a gradient: a forward, an adjoint and about one recompute or less, each launch
+    // of a segment with about 12 us of its own (state and m in and out)
+    const double seg = p->ckpt_every > 0 ? std::min(p->ckpt_every, p->nt) : std::max(1.0, std::sqrt((double)p->nt));
+    const double fwd = f->step_us + f->passes * 12.0 / seg, adj = a->step_us + a->passes * 12.0 / seg;
+    return 1.6 * fwd + adj < 0.95 * 2.6 * streamed;
+}
+
 // tile_rows > 0 overrides the problem's 2D tile height and step_block >= 1
 // its steps per launch (the u-store adjoint runs one step per launch on
 // 16-row tiles: its third staged tile must leave room for the stages).
-Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool vd = false) {
+Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool vd = false,
+               const ResPlan* rf = nullptr, const ResPlan* ra = nullptr) {
     Geom g{};
+    if (rf) {
+        g.res = true;
+        g.rf = *rf;
+        if (ra) g.ra = *ra;
+    }
     g.vd = vd;
     g.ndim = p->ndim;
     g.R = p->order / 2;
@@ -309,8 +344,12 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
     g.plane = (long long)g.ny * g.ld;
     g.cells = (long long)g.nz * g.plane;
     const int sb = step_block > 0 ? step_block : p->step_block;
-    g.sb = (p->ndim == 2 && (sb == 2 || (sb >= 4 && g.R * sb == WR_HALO))) ? sb : 1;
-    if (vd) {
+    g.sb = (p->ndim == 2 && !rf && (sb == 2 || (sb >= 4 && g.R * sb == WR_HALO))) ? sb : 1;
+    if (rf) {
+        g.tile_z = rf->tz;
+        g.tile_y = 1;
+        g.tile_x = RES_TX;
+    } else if (vd) {
         g.sb = 1;
         g.tile_z = 16;  // the variable-density kernel's 128 x 16 tile
         g.tile_y = 1;
@@ -390,6 +429,15 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
 
 // Geometry of the adjoint launches: 16-row tiles for the u-store adjoint.
 Geom adjoint_geom(const wfd_problem* p, const Geom& g) {
+    if (g.res) {
+        Geom a = g;
+        if (g.ra.rb > 0) {
+            a.tile_z = g.ra.tz;
+            a.tiles_z = g.ra.tiles_z;
+            a.ntiles = g.ra.ntiles;
+        }
+        return a;
+    }
     return g.ustore && (g.tile_z != 16 || g.sb != 1) ? make_geom(p, 16, 1) : g;
 }
 
@@ -404,6 +452,7 @@ struct Layout {
     size_t S[2], scale_bytes;  // reduced-precision fields: the int16 block scales
     size_t b, Gbx, Gbz;        // variable density: b = 1/rho, half-point gradient sums
     size_t frames, frame_bytes;  // reconstruction adjoint: the damped frame of u_1 .. u_nt
+    size_t mail;               // resident kernel: the tiles' mailboxes
     size_t D;                  // summed form: the increment field d_n (0: leapfrog)
     int nlap;  // slots of the lap region: K stored L u_k, or levels u_k (u store): from
                // u_{k0_store - 1} to u_nt, and at least K + 2 for a recomputed segment
@@ -484,6 +533,7 @@ Layout make_layout(const wfd_problem* p, const Geom& g, bool grad) {
         L.lap = take(std::max((size_t)L.nlap * L.lap_field_bytes, (size_t)L.nlvl * L.lvl_bytes));
         L.res = take((size_t)p->nshot * p->nt * p->nrec * 4 + 4);
     }
+    if (g.res) L.mail = take(std::max(g.rf.mail_bytes, grad ? g.ra.mail_bytes : 0));
     L.total = o;
     return L;
 }
@@ -493,6 +543,7 @@ struct Work {
     float *m, *P[4], *Q[4], *G, *res;
     float* S[2];  // int16 block scales of P[0], P[1] (reduced-precision fields)
     float *b, *Gbx, *Gbz;  // variable density (workspace)
+    void* mail;            // resident kernel: mailboxes
     float* D;              // summed form: the increment d_n, [nshot][cells] (null: leapfrog)
     const float* rho;      // variable density: the caller's rho, for setup and the gradient
     float* grad_rho;       // variable density: dJ/drho output
@@ -525,6 +576,7 @@ Work carve(void* ws, const Layout& L, bool grad) {
     }
     for (int k = 0; k < L.nbuf; ++k) w.P[k] = reinterpret_cast<float*>(b + L.P[k]);
     if (L.D) w.D = reinterpret_cast<float*>(b + L.D);
+    if (L.mail) w.mail = b + L.mail;
     if (L.S[0])
         for (int k = 0; k < 2; ++k) w.S[k] = reinterpret_cast<float*>(b + L.S[k]);
     w.counts = reinterpret_cast<int*>(b + L.counts);
@@ -565,6 +617,41 @@ int check_workspace(void* ws, size_t bytes, size_t need) {
     return WFD_OK;
 }
 
+// Whether the current device holds every CTA of a resident launch at once.
+bool resident_device() {
+    static std::atomic<int> known[64];  // per device: 0 not asked, 1 no, 2 yes
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int k = known[dev].load(std::memory_order_relaxed);
+    if (k == 0) {
+        int sms = 0, coop = 0, smem = 0;
+        const bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) == cudaSuccess &&
+                        sms >= RES_SMS && coop && smem >= RES_SMEM;
+        k = ok ? 2 : 1;
+        known[dev].store(k, std::memory_order_relaxed);
+    }
+    return k == 2;
+}
+
+// The geometry of a constant-density call: the resident kernel's where it runs
+// the problem and its layout fits the workspace given, else the streaming kernels'.
+// (A forward and its backward have to be given the same workspace size.)
+Geom call_geom(const wfd_problem* p, bool grad, size_t workspace_bytes) {
+    ResPlan f, a;
+    if (resident_plan(p, grad, &f, &a) && resident_device()) {
+        const Geom g = make_geom(p, 0, 0, false, &f, grad ? &a : nullptr);
+        if (make_layout(p, g, grad).total <= workspace_bytes) return g;
+    }
+    return make_geom(p);
+}
+
+// The geometry of a later shot group, which may be smaller than the first (gf).
+Geom group_geom(const wfd_problem* q, const Geom& gf) {
+    return gf.res ? make_geom(q, 0, 0, false, &gf.rf, gf.ra.rb > 0 ? &gf.ra : nullptr) : make_geom(q);
+}
+
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
 // ------------------------------------------------------------------ stepping
@@ -580,6 +667,7 @@ struct Stepper {
     const float* bfield = nullptr;  // variable density: b = 1/rho
 
     int init() {
+        if (g.res) return WFD_OK;
         if (g.vd) {  // b on the tile with R rows / 8 columns of halo (and one more row)
             EncodeTiled enc = encoder();
             if (!enc) return fail(WFD_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
@@ -806,9 +894,191 @@ int run_forward_reg(const wfd_problem* p, const Geom& g, const Layout& L, const 
     return WFD_OK;
 }
 
+// The resident kernel's launches (stencil2d_res.cuh) of one forward or backward:
+// every launch's tags lie above the last one's.
+struct Resident {
+    const wfd_problem* p;
+    const Work& w;
+    cudaStream_t s;
+    unsigned tag = 0;
+
+    int clear(size_t mail_bytes) {
+        WFD_CUDA(cudaMemsetAsync(w.mail, 0, mail_bytes, s));
+        return WFD_OK;
+    }
+    // every shot, as many at once as the plan holds
+    int launch(int R, ResMode mode, const ResPlan& plan, ResArgs& q) {
+        q.mail = w.mail;
+        for (int s0 = 0; s0 < p->nshot; s0 += plan.shots) {
+            q.shot0 = s0;
+            q.nshots = std::min(plan.shots, p->nshot - s0);
+            q.tag0 = tag;
+            tag += unsigned(q.steps);
+            const cudaError_t e = launch_resident(R, mode, plan, q, s);
+            if (e != cudaSuccess) return fail(WFD_ERR_CUDA, "resident launch failed: %s", cudaGetErrorString(e));
+        }
+        return WFD_OK;
+    }
+};
+
+// Forward on the resident kernel: one launch (per shots on the chip) advances a
+// whole checkpoint segment, or the whole forward without checkpoints. Level u_k
+// is P[k & 1] between launches; the kept segments leave L u_k, not u_k, in the
+// store's slots k - k0_store + 1, which is what the resident adjoint reads.
+int run_forward_res(const wfd_problem* p, const Geom& g, const Layout& L, const Work& w, const Stepper& st,
+                    const float* wavelet, float* traces, bool save, int* final_buf) {
+    cudaStream_t s = st.s;
+    const bool summed = summed_forward(p, g, save);
+    if (summed && !w.D) return fail(WFD_ERR_INVALID, "internal: summed forward without its increment field");
+    const ResMode mode = !summed ? RES_LEAP : p->step_block == 2 ? RES_SUMMED : RES_SUMMED_DIFF;
+    if (final_buf) *final_buf = p->nt & 1;
+    Resident run{p, w, s};
+    int rc = run.clear(g.rf.mail_bytes);
+    if (rc) return rc;
+    if (save && g.jstore > 0) {  // (the checkpoint of level 0)
+        WFD_CUDA(cudaMemsetAsync(w.P[0], 0, L.field_bytes, s));
+        WFD_CUDA(cudaMemsetAsync(summed ? w.D : w.P[1], 0, L.field_bytes, s));
+    }
+    const long long n_all = (long long)p->nshot * g.cells;
+    const int seg = save ? g.K : p->nt;
+    PhaseScope scope(PH_FORWARD, s, cdiv(p->nt, seg) * cdiv(p->nshot, g.rf.shots));
+    for (int n = 0; n < p->nt; n += seg) {
+        const int n1 = std::min(p->nt, n + seg);
+        float* other[2] = {summed ? w.D : w.P[(n + 1) & 1], summed ? w.D : w.P[(n1 + 1) & 1]};
+        if (save && n < g.k0_store) {
+            unsigned char* slot = w.ckpt + (size_t)(n / g.K) * 2 * L.ckpt_field_bytes;
+            WFD_CUDA(launch_pack(other[0], slot, n_all, p->ckpt_format, s));
+            WFD_CUDA(launch_pack(w.P[n & 1], slot + L.ckpt_field_bytes, n_all, p->ckpt_format, s));
+        }
+        ResArgs q{};
+        q.a = st.base(nullptr);
+        if (p->nsrc > 0) {
+            q.a.inj = w.src;
+            q.a.inj_val = wavelet;
+            q.a.inj_np = p->nsrc; q.a.inj_nt = p->nt;
+            q.a.inj_scale = p->src_scale;
+        }
+        if (traces && p->nrec > 0) {
+            q.a.smp = w.rec;
+            q.a.smp_out = traces;
+            q.a.smp_np = p->nrec; q.a.smp_nt = p->nt;
+            q.a.smp_scale = 1.f;
+        }
+        if (n > 0) {
+            q.u_in = w.P[n & 1];
+            q.x_in = other[0];
+        }
+        q.u_out = w.P[n1 & 1];
+        q.x_out = n1 < p->nt ? other[1] : nullptr;
+        if (save && n >= g.k0_store) {
+            q.lap = w.slot(L, n - g.k0_store + 1);
+            q.lap_stride = (long long)(L.lap_field_bytes / sizeof(float));
+        }
+        q.steps = n1 - n;
+        q.inj_t0 = n;
+        q.smp_t0 = n - 1;
+        q.dir = 1;
+        if ((rc = run.launch(g.R, mode, g.rf, q))) return rc;
+    }
+    if (traces && p->nrec > 0)
+        WFD_CUDA(launch_gather(w.P[p->nt & 1], g.cells, w.rec, g.ntiles, p->nshot, p->nrec, nullptr, 1.f, 0, traces,
+                               p->nt, p->nt - 1, s));
+    return WFD_OK;
+}
+
+// Adjoint on the resident kernel. A recomputed segment restores (u_{k0-1}, u_k0)
+// into P, advances them with L u_k written to slots k - k0 + 1, and the adjoint
+// sums q_{k+1} L u_k in registers over the segment; level q_k is Q[k & 1] between
+// launches.
+int run_backward_res(const wfd_problem* p, const Geom& g, const Layout& L, const Work& w, const Stepper& st,
+                     const float* wavelet, const float* dtraces, float* grad_vel, float* grad_wavelet,
+                     const float* vel, bool zero_G, bool finalize) {
+    cudaStream_t s = st.s;
+    const Geom ga = adjoint_geom(p, g);
+    const bool summed = summed_forward(p, g, true);  // the checkpoints hold (d_k0, u_k0)
+    Resident run{p, w, s};
+    int rc = run.clear(std::max(g.rf.mail_bytes, g.ra.mail_bytes));
+    if (rc) return rc;
+    if (zero_G) WFD_CUDA(cudaMemsetAsync(w.G, 0, (size_t)g.cells * 4, s));
+    const long long n_all = (long long)p->nshot * g.cells;
+    const long long slot = (long long)(L.lap_field_bytes / sizeof(float));
+    Stepper sa = st;
+    sa.g = ga;
+    for (int j = g.nseg - 1; j >= 0; --j) {
+        const int k0 = j * g.K, k1 = std::min(p->nt, k0 + g.K);
+        const int hi = k1 == p->nt ? p->nt : k1 - 1, lo = std::max(k0, 1);
+        if (hi < lo) break;  // (segment [0, 1): u_0 = 0)
+        if (j < g.jstore) {
+            PhaseScope scope(PH_RECOMPUTE, s, cdiv(p->nshot, g.rf.shots));
+            const unsigned char* ck = w.ckpt + (size_t)j * 2 * L.ckpt_field_bytes;
+            float *u = w.P[k0 & 1], *old = w.P[(k0 + 1) & 1];
+            WFD_CUDA(launch_unpack(ck + L.ckpt_field_bytes, u, n_all, p->ckpt_format, s));
+            if (summed)  // u_{k0-1} = u_k0 - d_k0
+                WFD_CUDA(launch_unpack_diff(ck, u, old, n_all, p->ckpt_format, s));
+            else
+                WFD_CUDA(launch_unpack(ck, old, n_all, p->ckpt_format, s));
+            ResArgs q{};
+            q.a = st.base(nullptr);
+            if (p->nsrc > 0) {
+                q.a.inj = w.src;
+                q.a.inj_val = wavelet;
+                q.a.inj_np = p->nsrc; q.a.inj_nt = p->nt;
+                q.a.inj_scale = p->src_scale;
+            }
+            q.u_in = u;
+            q.x_in = old;
+            q.lap = w.slot(L, 1);
+            q.lap_stride = slot;
+            q.steps = k1 - k0;
+            q.inj_t0 = k0;
+            q.smp_t0 = -1;
+            q.dir = 1;
+            if ((rc = run.launch(g.R, RES_LEAP, g.rf, q))) return rc;
+        }
+        PhaseScope scope(PH_ADJOINT, s, cdiv(p->nshot, g.ra.shots));
+        ResArgs q{};
+        q.a = sa.base(nullptr);
+        q.a.grad = w.G;
+        if (p->nrec > 0) {
+            q.a.inj = w.rec_a;
+            q.a.inj_val = dtraces;
+            q.a.inj_np = p->nrec; q.a.inj_nt = p->nt;
+            q.a.inj_scale = 1.f;
+            q.a.inj_times_m = 1;
+        }
+        if (grad_wavelet && p->nsrc > 0) {
+            q.a.smp = w.src_a;
+            q.a.smp_out = grad_wavelet;
+            q.a.smp_np = p->nsrc; q.a.smp_nt = p->nt;
+            q.a.smp_scale = p->src_scale;
+            q.a.smp_div_m = 1;
+        }
+        if (hi < p->nt) {  // (q_{nt+1} = q_{nt+2} = 0)
+            q.u_in = w.Q[(hi + 1) & 1];
+            q.x_in = w.Q[hi & 1];
+        }
+        q.u_out = w.Q[lo & 1];
+        q.x_out = w.Q[(lo + 1) & 1];
+        q.lap = w.slot(L, j < g.jstore ? hi - k0 + 1 : hi - g.k0_store + 1);
+        q.lap_stride = -slot;
+        q.lap_from = hi == p->nt ? 1 : 0;  // q_nt's gradient term is 0
+        q.steps = hi - lo + 1;
+        q.inj_t0 = hi - 1;
+        q.smp_t0 = hi;
+        q.dir = -1;
+        if ((rc = run.launch(g.R, RES_ADJOINT, g.ra, q))) return rc;
+    }
+    if (grad_wavelet && p->nsrc > 0)  // q_1 at the sources -> d J / d w_0
+        WFD_CUDA(launch_gather(w.Q[1], ga.cells, w.src_a, ga.ntiles, p->nshot, p->nsrc, w.m, p->src_scale, 1,
+                               grad_wavelet, p->nt, 0, s));
+    if (finalize) WFD_CUDA(launch_grad_finalize(w.G, vel, grad_vel, g.nz, g.ny, g.nx, g.ld, g.R, s));
+    return WFD_OK;
+}
+
 int run_forward(const wfd_problem* p, const Geom& g, const Layout& L, const Work& w,
                 const Stepper& st, const float* wavelet, float* traces, bool save,
                 int* final_buf = nullptr) {
+    if (g.res) return run_forward_res(p, g, L, w, st, wavelet, traces, save, final_buf);
     if (g.sb >= 4) {
         if (save) return fail(WFD_ERR_INVALID, "step_block %d is a forward-only mode", g.sb);
         return run_forward_reg(p, g, L, w, st, wavelet, traces, final_buf);
@@ -1344,6 +1614,8 @@ int run_backward_recon(const wfd_problem* p, const Geom& g, const Layout& L, con
 int run_backward(const wfd_problem* p, const Geom& g, const Layout& L, const Work& w,
                  const Stepper& st, const float* wavelet, const float* dtraces, float* grad_vel,
                  float* grad_wavelet, const float* vel, bool zero_G = true, bool finalize = true) {
+    if (g.res)
+        return run_backward_res(p, g, L, w, st, wavelet, dtraces, grad_vel, grad_wavelet, vel, zero_G, finalize);
     if (g.recon) {
         if (!zero_G || !finalize)
             return fail(WFD_ERR_INVALID, "the reconstruction adjoint does not run in shot groups");
@@ -1467,8 +1739,31 @@ int wfd_workspace_bytes(const wfd_problem* p, int with_gradient, size_t* bytes) 
     const wfd_problem q = group_problem(p, 0);  // the workspace serves one group at a time
     const Geom g = make_geom(&q);
     *bytes = make_layout(&q, g, with_gradient != 0).total;
+    // room for the resident kernel's mailboxes (its other fields are among the streaming
+    // kernels'); level_format changes the level store alone, so both formats have it
+    wfd_problem r = q;
+    r.level_format = WFD_LEVEL_FP32;
+    ResPlan f, a;
+    if (resident_plan(&r, with_gradient != 0, &f, &a)) {
+        *bytes += up256(std::max(f.mail_bytes, with_gradient ? a.mail_bytes : 0));
+        if (q.level_format == WFD_LEVEL_FP32)  // (smaller tiles have longer point lists)
+            *bytes = std::max(*bytes, make_layout(&q, make_geom(&q, 0, 0, false, &f, with_gradient ? &a : nullptr),
+                                                  with_gradient != 0).total);
+    }
     return WFD_OK;
 }
+
+}  // extern "C"
+
+int forward_min_bytes(const wfd_problem* p, size_t* bytes) {
+    const int rc = check_problem(p);
+    if (rc) return rc;
+    const wfd_problem q = group_problem(p, 0);
+    *bytes = make_layout(&q, make_geom(&q), false).total;
+    return WFD_OK;
+}
+
+extern "C" {
 
 int wfd_forward(const wfd_problem* p, const float* vel, const float* sponge_z,
                 const float* sponge_y, const float* sponge_x, const float* wavelet,
@@ -1484,12 +1779,13 @@ int wfd_forward(const wfd_problem* p, const float* vel, const float* sponge_z,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // one layout, sized for a full group, serves every group
     const wfd_problem first = group_problem(p, 0);
-    const Layout L = make_layout(&first, make_geom(&first), save_checkpoints != 0);
+    const Geom gf = call_geom(&first, save_checkpoints != 0, workspace_bytes);
+    const Layout L = make_layout(&first, gf, save_checkpoints != 0);
     if ((rc = check_workspace(workspace, workspace_bytes, L.total))) return rc;
     const Work w = carve(workspace, L, save_checkpoints != 0);
     for (int g0 = 0; g0 < p->nshot; g0 += G) {
         const wfd_problem q = group_problem(p, g0);
-        const Geom g = make_geom(&q);
+        const Geom g = group_geom(&q, gf);
         if ((rc = setup(&q, g, w, vel, src + 3L * g0 * p->nsrc, rec + 3L * g0 * p->nrec, s, g0 == 0)))
             return rc;
         Stepper st{&q, g, s, w.err, w.m, sponge_z, p->ndim == 3 ? sponge_y : nullptr, sponge_x};
@@ -1510,7 +1806,7 @@ int wfd_forward_final(const wfd_problem* p, const float* vel, const float* spong
     if (rc) return rc;
     if (!u_final) return fail(WFD_ERR_INVALID, "u_final is NULL");
     if (group_size(p) < p->nshot) return fail(WFD_ERR_INVALID, "no shot groups with u_final");
-    const Geom g = make_geom(p);
+    const Geom g = call_geom(p, false, workspace_bytes);
     const Layout L = make_layout(p, g, false);
     if ((rc = check_workspace(workspace, workspace_bytes, L.total))) return rc;
     const Work w = carve(workspace, L, false);
@@ -1544,7 +1840,7 @@ int wfd_backward(const wfd_problem* p, const float* vel, const float* sponge_z,
     if (p->step_block >= 4) return fail(WFD_ERR_INVALID, "step_block %d is a forward-only mode", p->step_block);
     if (group_size(p) < p->nshot)
         return fail(WFD_ERR_INVALID, "wfd_backward cannot be split into shot groups");
-    const Geom g = make_geom(p);
+    const Geom g = call_geom(p, true, workspace_bytes);
     const Layout L = make_layout(p, g, true);
     if ((rc = check_workspace(workspace, workspace_bytes, L.total))) return rc;
     const Work w = carve(workspace, L, true);
@@ -1576,14 +1872,15 @@ int misfit_gradient_impl(const wfd_problem* p, const float* vel, const float* sp
     // one layout, sized for a full group, serves every group (the gradient
     // accumulator keeps its address across groups)
     const wfd_problem first = group_problem(p, 0);
-    const Layout L = make_layout(&first, make_geom(&first), true);
+    const Geom gf = call_geom(&first, true, workspace_bytes);
+    const Layout L = make_layout(&first, gf, true);
     if ((rc = check_workspace(workspace, workspace_bytes, L.total))) return rc;
     const Work w = carve(workspace, L, true);
     for (int g0 = 0; g0 < p->nshot; g0 += G) {
         // one group: forward with checkpoints, residual, adjoint; the gradient
         // and the misfit accumulate over the groups
         const wfd_problem q = group_problem(p, g0);
-        const Geom g = make_geom(&q);
+        const Geom g = group_geom(&q, gf);
         const int32_t* gsrc = src + 3L * g0 * p->nsrc;
         const int32_t* grec = rec + 3L * g0 * p->nrec;
         const float* gwav = wavelet + (long long)g0 * p->nt * p->nsrc;

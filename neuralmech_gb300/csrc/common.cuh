@@ -204,9 +204,9 @@ __device__ __forceinline__ float4 bfp4_decode(uint2 q, unsigned t) {
 // through the packed FP32x2 arithmetic of sm_100+, with the operations and
 // their order of the scalar form c0 u + sum_k cx_k (u_{x-k} + u_{x+k}) +
 // cz_k (u_{z-k} + u_{z+k}), accumulated k = 1 .. R with x before z.
-template <int R, int N>
+template <int R, int N, class Weights>  // Weights: c0p, cxp[], czp[] (StepArgs, or a copy of them)
 __device__ __forceinline__ float4 lap_row(const float4& lv, const float4& cv, const float4& rv,
-                                          const float4 (&V)[N], int C, const StepArgs& a) {
+                                          const float4 (&V)[N], int C, const Weights& a) {
     const float w[12] = {lv.x, lv.y, lv.z, lv.w, cv.x, cv.y, cv.z, cv.w, rv.x, rv.y, rv.z, rv.w};
     float2 lo = __fmul2_rn(a.c0p, make_float2(cv.x, cv.y));
     float2 hi = __fmul2_rn(a.c0p, make_float2(cv.z, cv.w));
@@ -238,9 +238,9 @@ __device__ __forceinline__ float4 lap_row(const float4& lv, const float4& cv, co
 // field is exact or nearly so in FP32, and the sum's rounding is relative to
 // the differences instead of to |u| times the centre weight. Packed FP32x2
 // pairs as lap_row.
-template <int R, int N>
+template <int R, int N, class Weights>
 __device__ __forceinline__ float4 lap_row_diff(const float4& lv, const float4& cv, const float4& rv,
-                                               const float4 (&V)[N], int C, const StepArgs& a) {
+                                               const float4 (&V)[N], int C, const Weights& a) {
     const float w[12] = {lv.x, lv.y, lv.z, lv.w, cv.x, cv.y, cv.z, cv.w, rv.x, rv.y, rv.z, rv.w};
     // minus the centre values: x - u as one packed add of -u (the negation is exact)
     const float2 nl = make_float2(-cv.x, -cv.y), nh = make_float2(-cv.z, -cv.w);

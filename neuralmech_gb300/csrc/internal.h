@@ -158,6 +158,62 @@ cudaError_t launch_step2d(int R, int mode, int tile_rows, const CUtensorMap& map
                           const CUtensorMap& map_old, const CUtensorMap& map_lap, const StepArgs& a,
                           cudaStream_t s, const CUtensorMap* map_lx = nullptr);
 
+// ---------------------------------------------------------------- 2D, fields resident on the chip
+// A tile is RES_TX x (rb nwg) cells of one shot: nwg warps of rb rows (stencil2d_res.cuh).
+constexpr int RES_TX = 128;
+// Threads of a CTA by mode and rows per warp: the two float4 per row and thread that
+// live across steps (state; in the adjoint also the gradient sum), about 36 registers
+// of vertical window and 50 more have to fit the 64 K registers of an SM.
+constexpr int res_threads(int mode, int rb) {
+    return mode == 3 ? (rb <= 2 ? 512 : rb <= 7 ? 384 : 256) : (rb <= 10 ? 512 : 384);
+}
+// Rows of a warp whose m may come from L2 instead of shared memory (the largest tiles).
+constexpr int res_l2_rows(int rb) { return rb >= 19 ? 6 : 0; }
+constexpr int RES_PTS = 256;       // injected points linked per tile (more are looked up in the list)
+constexpr int RES_SMS = 152;       // CTAs that are resident at once, one per SM
+constexpr int RES_SMEM = 227 * 1024;
+
+// Shared memory of a group besides u and m: sponge factors, points (24 B each), 4 B a thread.
+constexpr int res_group_bytes(int nwg, int tz) {
+    return 4 * RES_TX + (tz + 3) / 4 * 16 + 24 * RES_PTS + 32 + 128 * nwg;
+}
+
+enum ResMode : int { RES_LEAP = 0, RES_SUMMED = 1, RES_SUMMED_DIFF = 2, RES_ADJOINT = 3 };
+
+struct ResPlan {
+    int rb = 0;      // rows per warp (0: no plan)
+    int nwg = 0;     // warps per group
+    int ng = 0;      // groups (tiles) per CTA
+    int lm = 0;      // rows of a warp whose m comes from L2
+    int share_m = 0; // a CTA's groups hold the same tile of different shots
+    int tz = 0, tiles_z = 0, tiles_x = 0, ntiles = 0;
+    int shots = 0;   // shots on the chip at once
+    int passes = 0;  // launches that take every shot one stretch of steps further
+    size_t smem = 0, mail_bytes = 0;
+    double step_us = 0;  // estimated time of one step of all shots
+    int ctas(int n) const { return share_m ? ntiles * ((n + ng - 1) / ng) : (ntiles * n + ng - 1) / ng; }
+};
+
+// The split of nshot shots of an nz x nx grid over the chip with the least
+// estimated time; false when not even one shot fits.
+bool plan_resident(int nz, int nx, int R, int nshot, ResMode mode, ResPlan* out);
+
+struct ResArgs {
+    StepArgs a;               // geometry, weights, m, sponge, point lists, gradient sum (adjoint)
+    const float *u_in, *x_in; // the state: u_n and u_{n-1} (or d_n), [nshot][cells]; null: 0
+    float *u_out, *x_out;     // the state after the last step (null: not written)
+    float* lap;               // L u of the level at step it: lap + it lap_stride, from step lap_from
+    long long lap_stride;     //   on (forward: written when not null; adjoint: read, q L u summed)
+    int lap_from;
+    int steps;
+    int inj_t0, smp_t0, dir;  // injection and sample indices of step 0, and their increment
+    void* mail;               // mailboxes (mail_bytes, tags below tag0 + 1)
+    unsigned tag0;            // the launch uses tags tag0 + 1 .. tag0 + steps
+    int shot0, nshots;        // the shots of this launch
+    int nwg, ng, lm, share_m, tz, ntiles;
+};
+cudaError_t launch_resident(int R, ResMode mode, const ResPlan& plan, const ResArgs& q, cudaStream_t s);
+
 // ---------------------------------------------------------------- 2D, two steps per launch
 // Tile T = K2_TX x K2_TZ cells; u_n is staged on T plus 2R rows / 8 columns
 // (K2_UW wide), u_{n-1} and m on E = T plus R rows / 4 columns (K2_EW wide).

@@ -40,6 +40,10 @@
 #include "../../include/wavefd.h"
 #include "internal.h"
 
+// The least workspace of a forward without checkpoints (api.cu): less than
+// wfd_workspace_bytes where that has room for the resident kernel's mailboxes.
+int forward_min_bytes(const wfd_problem* p, size_t* bytes);
+
 namespace {
 
 constexpr size_t kStaticScratchBytes = size_t(64) << 20;
@@ -80,7 +84,7 @@ extern "C" int wfd_forward_static(const wfd_problem* p, const float* vel, const 
                                   const float* wavelet, const int32_t* src, const int32_t* rec,
                                   float* traces, void* stream) {
     size_t need = 0;
-    int rc = wfd_workspace_bytes(p, 0, &need);
+    int rc = forward_min_bytes(p, &need);
     if (rc) return rc;
     if (need > kStaticScratchBytes)
         return wfd::set_error(WFD_ERR_WORKSPACE,

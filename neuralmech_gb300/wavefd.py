@@ -61,11 +61,14 @@ class Grid:
              term: "auto" (2D one-step kernel: the level u_k, which the
              recompute writes anyway, with L u_k formed by the adjoint; else
              FP32 L u_k), "fp32" or "bf16" (L u_k stored in that type)
-    shots_per_cta  shots one CTA walks through per step (0 = automatic)
+    shots_per_cta  shots one CTA of a streaming kernel walks through per step (0 =
+             automatic; with tile_rows 0 also the resident kernel, which keeps
+             the fields of grids up to about 2048^2 on the chip, where faster)
     group_shots  run the shots of a misfit gradient (or of a forward without
              autograd) in sequential groups of this many, sharing one workspace
              sized for a group (0 = all at once)
-    tile_rows    2D tile height, 16 or 32 rows (0 = 32)
+    tile_rows    2D streaming tile height, 16 or 32 rows (0 = 32, or the resident
+             kernel)
     step_block   2D time steps per kernel launch, 1 or 2 (0 = 1); for a
              forward (no gradient) with the leapfrog update and FP32 fields
              also 8 at order 2 or 4 at order 4 (a register window per CTA)

@@ -4,6 +4,7 @@
 // work is in stencil2d.cu / stencil3d.cu / aux.cu.
 #include <nvtx3/nvToolsExt.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <map>
@@ -323,7 +324,7 @@ bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
     return 1.6 * fwd + adj < 0.95 * 2.6 * streamed;
 }
 
-// tile_rows > 0 overrides the problem's 2D tile height and step_block >= 1
+// tile_rows > 0 overrides the problem's 2D tile height (3D: the planes per CTA) and step_block >= 1
 // its steps per launch (the u-store adjoint runs one step per launch on
 // 16-row tiles: its third staged tile must leave room for the stages).
 Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool vd = false,
@@ -371,7 +372,8 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
         g.tile_y = 1;
         g.tile_x = T2_TX;
     } else {
-        g.tile_z = T3_ZCHUNK; g.tile_y = T3_TY; g.tile_x = T3_TX;
+        g.tile_z = tile_rows > 0 ? tile_rows : plan_zchunk3d(g.nz, g.ny, g.nx, p->nshot);
+        g.tile_y = T3_TY; g.tile_x = T3_TX;
     }
     g.tiles_z = cdiv(g.nz, g.tile_z);
     g.tiles_y = cdiv(g.ny, g.tile_y);
@@ -644,11 +646,16 @@ Geom call_geom(const wfd_problem* p, bool grad, size_t workspace_bytes) {
         const Geom g = make_geom(p, 0, 0, false, &f, grad ? &a : nullptr);
         if (make_layout(p, g, grad).total <= workspace_bytes) return g;
     }
+    if (p->ndim == 3) {  // (shorter columns have longer point lists)
+        const Geom g = make_geom(p);
+        return make_layout(p, g, grad).total <= workspace_bytes ? g : make_geom(p, T3_ZCHUNK);
+    }
     return make_geom(p);
 }
 
 // The geometry of a later shot group, which may be smaller than the first (gf).
 Geom group_geom(const wfd_problem* q, const Geom& gf) {
+    if (gf.ndim == 3) return make_geom(q, gf.tile_z);
     return gf.res ? make_geom(q, 0, 0, false, &gf.rf, gf.ra.rb > 0 ? &gf.ra : nullptr) : make_geom(q);
 }
 
@@ -719,6 +726,7 @@ struct Stepper {
         a.nshot = p->nshot;
         a.shots_per_cta = g.spc;
         a.tiles_x = g.tiles_x; a.tiles_y = g.tiles_y; a.tiles_z = g.tiles_z;
+        a.tile_z = g.tile_z;
         a.c0 = g.c0;
         for (int k = 0; k < 4; ++k) { a.cz[k] = g.cz[k]; a.cy[k] = g.cy[k]; a.cx[k] = g.cx[k]; }
         a.zero_ring = 1;  // the wave path's ring is 0 in every level
@@ -1739,6 +1747,7 @@ int wfd_workspace_bytes(const wfd_problem* p, int with_gradient, size_t* bytes) 
     const wfd_problem q = group_problem(p, 0);  // the workspace serves one group at a time
     const Geom g = make_geom(&q);
     *bytes = make_layout(&q, g, with_gradient != 0).total;
+    if (q.ndim == 3) *bytes = std::max(*bytes, make_layout(&q, make_geom(&q, T3_ZCHUNK), with_gradient != 0).total);
     // room for the resident kernel's mailboxes (its other fields are among the streaming
     // kernels'); level_format changes the level store alone, so both formats have it
     wfd_problem r = q;
@@ -1759,7 +1768,7 @@ int forward_min_bytes(const wfd_problem* p, size_t* bytes) {
     const int rc = check_problem(p);
     if (rc) return rc;
     const wfd_problem q = group_problem(p, 0);
-    *bytes = make_layout(&q, make_geom(&q), false).total;
+    *bytes = make_layout(&q, make_geom(&q, q.ndim == 3 ? T3_ZCHUNK : 0), false).total;
     return WFD_OK;
 }
 

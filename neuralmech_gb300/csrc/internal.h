@@ -67,6 +67,7 @@ struct StepArgs {
     long long shot_stride;     // cells per shot (nz * plane)
     int nshot, shots_per_cta;
     int tiles_x, tiles_y, tiles_z;
+    int tile_z;                // 3D: output planes per CTA (at most T3_ZCHUNK)
     float c0;                  // centre weight (all axes)
     float cz[4], cy[4], cx[4]; // axis weights for k = 1..R, already scaled by (dx/h)^2
     float2 c0p, czp[4], cyp[4], cxp[4]; // the same as duplicated pairs, operands of the
@@ -292,7 +293,14 @@ constexpr int T3_XH = 4;
 constexpr int T3_W = T3_TX + 2 * T3_XH;
 constexpr int T3_ROWS = 1;                       // tile rows per thread
 constexpr int T3_THREADS = (T3_TX / 4) * T3_TY / T3_ROWS;
-constexpr int T3_ZCHUNK = 64;                    // planes per CTA (z blocking)
+constexpr int T3_ZCHUNK = 64;                    // planes per CTA at most (z blocking)
+
+// Planes per CTA. A CTA spends about 6 planes' time on filling its queues and rings,
+// so a large grid takes T3_ZCHUNK; a small one takes what fills the chip's two CTAs
+// per SM with the fewest planes in a row. Measured, us a step at 64 planes / planned:
+// 64^3 98 / 20 (8 planes), 2 shots of 97 x 131 x 149 50 / 24 (20), 160^3 51 / 21 (8),
+// gradient of 4 shots of 144 x 128 x 160 68 / 52 per launch (48).
+int plan_zchunk3d(int nz, int ny, int nx, int nshot);
 
 // map_cur: u_n planes (box T3_W x (T3_TY + 2R) x 1 x 1); map_old, map_lap:
 // output-plane tiles (box T3_TX x T3_TY x 1 x 1); map_m: the model m

@@ -5,7 +5,8 @@
 // on fields [shot][z][y][ld] FP32 (x fastest, ld a multiple of 8).
 //
 // Per CTA (256 threads = 16 lanes along x x 16 rows along y): one shot, one
-// 64 x 16 (x, y) column, marching along z through T3_ZCHUNK output planes.
+// 64 x 16 (x, y) column, marching along z through a.tile_z output planes (at most
+// T3_ZCHUNK; fewer on small grids, chosen by plan_zchunk3d).
 // The shot is the fastest grid index: the CTAs of all shots of one column run
 // together, so m and (MODE_GRAD) the gradient tile are read from DRAM once
 // per column and served from L2 to the other shots.
@@ -80,8 +81,8 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
     const int tx_i = tile % a.tiles_x;
     const int ty_i = (tile / a.tiles_x) % a.tiles_y;
     const int tz_i = tile / (a.tiles_x * a.tiles_y);
-    const int x0 = tx_i * T3_TX, y0 = ty_i * T3_TY, z0 = tz_i * T3_ZCHUNK;
-    const int zc = min(T3_ZCHUNK, a.nz - z0);  // output planes of this CTA
+    const int x0 = tx_i * T3_TX, y0 = ty_i * T3_TY, z0 = tz_i * a.tile_z;
+    const int zc = min(a.tile_z, a.nz - z0);  // output planes of this CTA
     const int total = zc + 2 * R;               // u_n planes it stages
 
     const uint32_t lap_bytes = MODE == MODE_GRAD ? uint32_t(T3_TY * T3_TX * (a.lap_bf16 ? 2 : 4)) : 0u;
@@ -109,8 +110,11 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
         fence_mbar_init();
     }
     __syncthreads();
-    if (tid == 0)
+    grid_dependency_wait();  // (a programmatic dependent: every global access comes after this)
+    if (tid == 0) {
         for (int p = 0; p < min(NB, total); ++p) issue(p);
+        launch_dependents();
+    }
     if (tid < zc) gzs[tid] = a.gz != nullptr ? __ldg(a.gz + z0 + tid) : 1.f;
 
     // ---- per-thread constants
@@ -337,9 +341,10 @@ cudaError_t launch_impl(const CUtensorMap& mc, const CUtensorMap& mo, const CUte
         configured_device = dev;
     }
     const dim3 grid(a.nshot, a.tiles_x * a.tiles_y * a.tiles_z);
-    step3d_kernel<R, MODE, T3_ROWS><<<grid, T3_THREADS, L::BYTES, s>>>(mc, mo, ml, mm, with_weight_pairs(a));
+    const cudaError_t e = launch_pdl(step3d_kernel<R, MODE, T3_ROWS>, grid, dim3(T3_THREADS), L::BYTES, s, mc, mo, ml, mm,
+                                     with_weight_pairs(a));
     count_launch();
-    return cudaGetLastError();
+    return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 template <int R>
@@ -357,6 +362,26 @@ cudaError_t dispatch(int mode, const CUtensorMap& mc, const CUtensorMap& mo, con
 }  // namespace
 
 bool step3d_available() { return true; }
+
+int plan_zchunk3d(int nz, int ny, int nx, int nshot) {
+    const long long columns = (long long)((ny + T3_TY - 1) / T3_TY) * ((nx + T3_TX - 1) / T3_TX) * nshot;
+    int best = T3_ZCHUNK;
+    double least = 0;
+    for (int n = (nz + T3_ZCHUNK - 1) / T3_ZCHUNK; n <= nz; ++n) {
+        const int chunk = (nz + n - 1) / n;
+        const long long ctas = columns * ((nz + chunk - 1) / chunk), slots = 2 * 152;
+        if (n > (nz + T3_ZCHUNK - 1) / T3_ZCHUNK && (chunk < 4 || ctas > 65535)) break;
+        // a lone CTA of an SM takes about 0.7 of the time of two for a plane
+        const double waves = ctas <= slots / 2 ? 0.7 : ctas < 4 * slots ? double((ctas + slots - 1) / slots)
+                                                                      : double(ctas) / slots + 0.5;
+        const double t = waves * (chunk + 6.0);
+        if (least == 0 || t < least) {
+            least = t;
+            best = chunk;
+        }
+    }
+    return best;
+}
 
 cudaError_t launch_step3d(int R, int mode, const CUtensorMap& mc, const CUtensorMap& mo,
                           const CUtensorMap& ml, const CUtensorMap& mm, const StepArgs& a,

@@ -107,6 +107,13 @@ using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, 
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiled encoder() {
+    // cuTensorMapEncodeTiled wants a current context, and a thread that has made no
+    // runtime call yet (autograd's, on a first backward) has none
+    thread_local bool bound = false;
+    if (!bound) {
+        int dev = 0;
+        bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+    }
     static EncodeTiled fn = nullptr;
     if (!fn) {
         void* p = nullptr;

@@ -2164,8 +2164,8 @@ int wfd_temporal_step_fast(const float* u0, const float* u1, float* v0, float* v
     };
     if (overlap(v0, u0) || overlap(v0, u1) || overlap(v1, u0) || overlap(v1, u1) || overlap(v0, v1))
         return fail(WFD_ERR_INVALID, "v0 and v1 must not overlap each other, u0 or u1");
-    const cudaError_t e = launch_temporal_reg(u0, u1, v0, v1, wavespeed, dt, dx, dy, N, M, M_padded, false,
-                                              static_cast<cudaStream_t>(stream));
+    const cudaError_t e = launch_temporal_stream(u0, u1, v0, v1, wavespeed, dt, dx, dy, N, M, M_padded,
+                                                 static_cast<cudaStream_t>(stream));
     if (e != cudaSuccess) return fail(WFD_ERR_CUDA, "temporal step launch failed: %s", cudaGetErrorString(e));
     return WFD_OK;
 }

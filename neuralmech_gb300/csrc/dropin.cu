@@ -13,6 +13,8 @@
 // The reference's row index i runs with dx and its column index j (fastest,
 // M of them, padded to M_padded) with dy. Rows 0 and N - 1 and columns 0 and
 // M - 1 are the fixed boundary.
+#include <algorithm>
+
 #include "../../include/wavefd.h"
 #include "common.cuh"
 #include "internal.h"
@@ -284,122 +286,158 @@ __global__ void __launch_bounds__(TT_THREADS)
     }
 }
 
-// Eight steps per launch with the window in registers (temporal_step's
-// arguments and results). A CTA of 8 warps holds a 256-column x 40-row window:
-// thread t owns column t, both levels of its 40 rows in registers. The
-// vertical neighbours are registers of the same thread, the horizontal ones
-// come from the neighbouring lanes by warp shuffles; at a warp's edge, lane 0
-// and lane 31 read the neighbouring warp's edge column, which every warp
-// publishes in shared memory at each step (double-buffered by step parity:
-// one CTA barrier per step). The halo is 8 cells on every side, so the
-// 240 x 24 inner tile is exact after the eight steps; the global boundary is
-// never updated, as in temporal_step. Each cell is
-// loaded and stored once per launch with coalesced row accesses (a warp reads
-// 128 contiguous bytes of a row).
-//   EXACT: the reference expression in IEEE operations (update2d), value for
-//          value the reference's padded_step applied eight times;
-//   else:  u_{n+1} = (2 u - u_{n-1}) + cx (u_{i-1} - 2u + u_{i+1}) + cy (...),
-//          cx = k / dx^2, cy = k / dy^2 (fused multiply-adds, no division):
-//          within FP32 rounding of the reference, as its own --use_fast_math
-//          build (approximate division) is.
-constexpr int TR_NW = 8;                    // warps per CTA
-constexpr int TR_W = 32 * TR_NW;            // window columns, one per thread
-constexpr int TR_H = 40;                    // window rows held by each thread
-constexpr int TR_MINB = 2;                  // resident CTAs per SM the register budget allows
-constexpr int TR_HALO = 8;                  // = steps per launch
-constexpr int TR_OX = TR_W - 2 * TR_HALO;   // 240 output columns per CTA
+// Eight steps per launch as a stream of rows (temporal_step's arguments and results,
+// pre-divided weights and fused multiply-adds).
+//
+// A warp marches down a strip of 128 columns, 4 per lane, and carries all eight steps
+// along: at row t it takes u_n there and u_{n-1}, forms u_{n+1} of row t - 1, from that
+// u_{n+2} of row t - 2, and so on to u_{n+8} of row t - 8. Per step it keeps the row
+// above (prev) and the two parts of the next row's result that do not need the row below:
+//   u = Q + cx (S + v),                                           (row t - s - 1 done)
+//   Q = (2 v - old) + cy ((l - 2 v) + r),  S = prev - 2 v,        (row t - s begun)
+// with old the level two before at row t - s, which is the prev that the step before has
+// just replaced. The neighbours l and r of a lane's 4 cells are two shuffles; nothing is
+// exchanged between warps, so there is neither shared state nor a barrier. A step spreads
+// what a strip's edge does not know by one column and one row: the stored columns lie
+// TS_HALO inside the strip, and a warp starts TS_HALO rows above its first stored row.
+//
+// Why this form: the window kernel it replaces (256 x 40 cells in registers, 240 x 24 of
+// them stored) computed 1.8 times the cells stored and met at a CTA barrier per step. Here
+// it is 128 / 112 in x and (rows + 16) / rows in z. Rows come through a ring of 16-byte
+// asynchronous copies that only the copying lane reads. 8000 x 16000: 1243 -> 463 us a
+// launch (823 -> 2210 G updates/s, 4.4 TB/s of the 16 bytes a launch moves per cell), the
+// same values; what bounds it now is issue at 12 warps per SM (the state of eight steps,
+// 96 registers, leaves no room for more; folding S into Q saves 32 of them and 40 us, for
+// 18% more rounding error).
+//
+// The fixed cells (rows 0 and N - 1, columns 0 and M - 1, and what lies outside) keep the
+// value of two levels before; only warps that meet them (EDGE) look.
+constexpr int TS_STEPS = 8, TS_HALO = 8;
+constexpr int TS_COLS = 128 - 2 * TS_HALO;  // stored columns of a strip
+constexpr int TS_WARPS = 4;                 // warps of a CTA (independent)
+constexpr int TS_RING = 6;                  // rows in flight per warp
 
-// One step on the window: old <- the new level from (old, cur). GUARD: test
-// every cell against the shrinking window and the global boundary (CTAs whose
-// window reaches the boundary). Without it (windows inside the interior),
-// every cell but the window's first and last rows is updated: the window's
-// edge cells then take values from missing neighbours, but after s steps
-// those spread s cells inwards at most, and the stored tile lies 8 cells in.
-template <bool EXACT, bool GUARD, int H>
-__device__ __forceinline__ void reg_step(float (&old)[H], const float (&cur)[H], float (*edge)[2][H], int warp,
-                                         int lane, bool cupd, int rmin, int rmax, float k, float dx2, float dy2,
-                                         float cx, float cy) {
-    if (lane == 0 || lane == 31) {  // this warp's edge column, for the neighbouring warps
-        float* dst = edge[warp][lane == 31 ? 1 : 0];
+template <bool VEC, bool CHECK>
+__device__ __forceinline__ void copy_row(float* dst, const float* src, bool row_in, int j, int M) {
+    const unsigned d = smem_addr(dst);
+    if (VEC) {  // (j is a multiple of 4 and the rows are whole groups of 4: inside the row for j < M)
+        const int n = !CHECK || (row_in && j >= 0 && j < M) ? 16 : 0;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    } else {
 #pragma unroll
-        for (int r = 0; r < H; ++r) dst[r] = cur[r];
-    }
-    __syncthreads();
-    // lane 0: the previous warp's lane-31 column; lane 31: the next warp's
-    // lane-0 column (the window's outer columns are never updated)
-    const float* nb = lane == 31 ? edge[min(warp + 1, TR_NW - 1)][0] : edge[max(warp - 1, 0)][1];
-#pragma unroll
-    for (int r = 1; r < H - 1; ++r) {
-        const float c = cur[r];
-        float l = __shfl_up_sync(0xffffffffu, c, 1);
-        float rr = __shfl_down_sync(0xffffffffu, c, 1);
-        const float e = nb[r];
-        if (lane == 0) l = e;
-        if (lane == 31) rr = e;
-        if (!GUARD || (cupd && r > rmin && r < rmax)) {
-            if (EXACT) {
-                old[r] = update2d(old[r], c, cur[r - 1], cur[r + 1], l, rr, k, dx2, dy2);
-            } else {
-                const float two_c = 2.f * c;
-                old[r] = fmaf(cx, (cur[r - 1] - two_c) + cur[r + 1], fmaf(cy, (l - two_c) + rr, two_c - old[r]));
-            }
+        for (int e = 0; e < 4; ++e) {
+            const int n = !CHECK || (row_in && j + e >= 0 && j + e < M) ? 4 : 0;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + 4 * e), "l"(src + e), "r"(n) : "memory");
         }
     }
 }
 
-// H window rows per thread (H - 16 output rows per CTA), MINB resident CTAs
-// per SM for the register allocation.
-template <bool EXACT, int H, int MINB>
-__global__ void __launch_bounds__(TR_W, MINB)
-    temporal_reg_kernel(const float* __restrict__ u0, const float* __restrict__ u1, float* __restrict__ v0,
-                        float* __restrict__ v1, float k, float dx2, float dy2, float cx, float cy, int N, int M,
-                        int Mp) {
-    __shared__ float edge[2][TR_NW][2][H];  // [step parity][warp][lane 0 / lane 31][row]
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int j = blockIdx.x * TR_OX - TR_HALO + t;
-    const int i0 = blockIdx.y * (H - 2 * TR_HALO) - TR_HALO;
-    const bool jin = j >= 0 && j < M;
-    float A[H], B[H];  // u_{n-1}, u_n; they trade roles every step
+template <bool VEC>
+__global__ void __launch_bounds__(32 * TS_WARPS, 3)
+    temporal_stream_kernel(const float* __restrict__ u0, const float* __restrict__ u1, float* __restrict__ v0,
+                           float* __restrict__ v1, float cx, float cy, int N, int M, int Mp, int strips, int rows) {
+    __shared__ __align__(16) float ring[TS_WARPS][TS_RING][2][128];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int id = blockIdx.x * TS_WARPS + warp;
+    const int j = id % strips * TS_COLS - TS_HALO + 4 * lane;
+    const int z0 = id / strips * rows, z1 = min(N, z0 + rows);
+    if (z0 >= N) return;
+    float* own = &ring[warp][0][0][4 * lane];
+    auto march = [&](auto edge_c) {
+        constexpr bool EDGE = decltype(edge_c)::value;
+        bool fixed[4];  // columns that keep their values
 #pragma unroll
-    for (int r = 0; r < H; ++r) {
-        const int i = i0 + r;
-        const bool in = jin && i >= 0 && i < N;  // cells outside the grid hold 0
-        const long long c = (long long)i * Mp + j;
-        A[r] = in ? __ldg(u0 + c) : 0.f;
-        B[r] = in ? __ldg(u1 + c) : 0.f;
-    }
-    const bool jupd = j > 0 && j < M - 1;  // the boundary columns (and beyond) stay untouched
-    const int j0 = blockIdx.x * TR_OX - TR_HALO;
-    const bool inner = i0 >= 1 && i0 + H - 1 <= N - 2 && j0 >= 1 && j0 + TR_W - 1 <= M - 2;  // (CTA-uniform)
-    for (int st = 0; st < TR_HALO; st += 2) {
-        if (inner) {
-            reg_step<EXACT, false, H>(A, B, edge[0], warp, lane, true, 0, 0, k, dx2, dy2, cx, cy);
-            reg_step<EXACT, false, H>(B, A, edge[1], warp, lane, true, 0, 0, k, dx2, dy2, cx, cy);
-            continue;
-        }
-        // updated rows: inside the shrinking window and inside (0, N - 1)
-        for (int h = 0; h < 2; ++h) {
-            const int s2 = st + h;
-            const int rmin = max(s2, -i0), rmax = min(H - 1 - s2, N - 1 - i0);
-            const bool cupd = jupd && t > s2 && t < TR_W - 1 - s2;
-            if (h == 0)
-                reg_step<EXACT, true, H>(A, B, edge[0], warp, lane, cupd, rmin, rmax, k, dx2, dy2, cx, cy);
-            else
-                reg_step<EXACT, true, H>(B, A, edge[1], warp, lane, cupd, rmin, rmax, k, dx2, dy2, cx, cy);
-        }
-    }
-    // A holds u_{n+7}, B u_{n+8}
-    if (t >= TR_HALO && t < TR_W - TR_HALO && j < M) {
+        for (int e = 0; e < 4; ++e) fixed[e] = j + e <= 0 || j + e >= M - 1;
+        const float2 cx2 = make_float2(cx, cx), cy2 = make_float2(cy, cy);
+        const float2 mone = make_float2(-1.f, -1.f), mtwo = make_float2(-2.f, -2.f);
+        float4 Q[TS_STEPS], S[TS_STEPS], prev[TS_STEPS];
 #pragma unroll
-        for (int r = TR_HALO; r < H - TR_HALO; ++r) {
-            const int i = i0 + r;
-            if (i < N) {
-                const long long c = (long long)i * Mp + j;
-                v0[c] = A[r];
-                v1[c] = B[r];
+        for (int s = 0; s < TS_STEPS; ++s) Q[s] = S[s] = prev[s] = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int first = z0 - TS_HALO, last = z1 - 1 + TS_STEPS;
+        // row t into the ring; what lies outside the grid (only EDGE warps meet it) as zeros
+        const float *p0 = u0 + ((long long)first * Mp + j), *p1 = u1 + ((long long)first * Mp + j);
+        int next = first;
+        auto fetch = [&](int slot) {
+            if (EDGE) {
+                const bool in = next >= 0 && next < N;
+                copy_row<VEC, true>(own + slot * 256, in && j < M ? p0 : u0, in, j, M);
+                copy_row<VEC, true>(own + slot * 256 + 128, in && j < M ? p1 : u1, in, j, M);
+            } else if (next <= last) {
+                copy_row<VEC, false>(own + slot * 256, p0, true, j, M);
+                copy_row<VEC, false>(own + slot * 256 + 128, p1, true, j, M);
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            ++next;
+            p0 += Mp;
+            p1 += Mp;
+        };
+        for (int k = 0; k < TS_RING; ++k) fetch(k);
+        float *o0 = v0 + ((long long)(first - 7) * Mp + j), *o1 = v1 + ((long long)(first - 8) * Mp + j);
+        const bool stores = lane >= TS_HALO / 4 && lane < 32 - TS_HALO / 4;
+        int slot = 0;
+        // (four rows per turn: the values handed from a step to the next then change registers by name)
+#pragma unroll 4
+        for (int t = first; t <= last; ++t) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(TS_RING - 1) : "memory");
+            float4 old = *reinterpret_cast<const float4*>(own + slot * 256);
+            float4 v = *reinterpret_cast<const float4*>(own + slot * 256 + 128);
+            fetch(slot);
+            slot = slot + 1 == TS_RING ? 0 : slot + 1;
+            float4 seventh;
+#pragma unroll
+            for (int s = 0; s < TS_STEPS; ++s) {
+                // (differences as multiply-adds by -1 and -2, which are exact: a packed add
+                // would negate its operand first)
+                const float4 p = prev[s], q = Q[s], c = S[s];
+                const float2 vl = make_float2(v.x, v.y), vh = make_float2(v.z, v.w);
+                float2 ul = __ffma2_rn(cx2, __fadd2_rn(make_float2(c.x, c.y), vl), make_float2(q.x, q.y));
+                float2 uh = __ffma2_rn(cx2, __fadd2_rn(make_float2(c.z, c.w), vh), make_float2(q.z, q.w));
+                const float l = __shfl_up_sync(0xffffffffu, v.w, 1), r = __shfl_down_sync(0xffffffffu, v.x, 1);
+                const float2 dl = __fadd2_rn(__ffma2_rn(mtwo, vl, make_float2(l, v.x)), make_float2(v.y, v.z));
+                const float2 dh = __fadd2_rn(__ffma2_rn(mtwo, vh, make_float2(v.y, v.z)), make_float2(v.w, r));
+                float2 ql = __ffma2_rn(cy2, dl, __ffma2_rn(mone, make_float2(old.x, old.y), __fadd2_rn(vl, vl)));
+                float2 qh = __ffma2_rn(cy2, dh, __ffma2_rn(mone, make_float2(old.z, old.w), __fadd2_rn(vh, vh)));
+                const float2 sl = __ffma2_rn(mtwo, vl, make_float2(p.x, p.y)), sh = __ffma2_rn(mtwo, vh, make_float2(p.z, p.w));
+                if (EDGE) {
+                    // fixed cells: Q holds old, and the finished row takes Q as it is
+                    const bool row = t - s <= 0 || t - s >= N - 1, above = t - s - 1 <= 0 || t - s - 1 >= N - 1;
+                    ql.x = row || fixed[0] ? old.x : ql.x;
+                    ql.y = row || fixed[1] ? old.y : ql.y;
+                    qh.x = row || fixed[2] ? old.z : qh.x;
+                    qh.y = row || fixed[3] ? old.w : qh.y;
+                    ul.x = above || fixed[0] ? q.x : ul.x;
+                    ul.y = above || fixed[1] ? q.y : ul.y;
+                    uh.x = above || fixed[2] ? q.z : uh.x;
+                    uh.y = above || fixed[3] ? q.w : uh.y;
+                }
+                Q[s] = make_float4(ql.x, ql.y, qh.x, qh.y);
+                S[s] = make_float4(sl.x, sl.y, sh.x, sh.y);
+                prev[s] = v;
+                old = p;
+                v = make_float4(ul.x, ul.y, uh.x, uh.y);
+                if (s == TS_STEPS - 2) seventh = v;  // u_{n+7} of row t - 7; v ends as u_{n+8} of row t - 8
+            }
+            auto put = [&](float* o, const float4& u) {
+                if (VEC && (!EDGE || j + 3 < M)) {
+                    __stcs(reinterpret_cast<float4*>(o), u);
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (j + e < M) o[e] = comp(u, e);
+                }
+            };
+            if (stores && t >= z0 + 7 && t < z1 + 7) put(o0, seventh);
+            if (stores && t >= z0 + 8) put(o1, v);
+            o0 += Mp;
+            o1 += Mp;
         }
-    }
+        asm volatile("cp.async.wait_all;" ::: "memory");
+    };
+    const int j0 = id % strips * TS_COLS - TS_HALO;
+    if (j0 <= 0 || j0 + 128 >= M || z0 - TS_HALO <= 0 || z1 + TS_HALO >= N)
+        march(Flag<true>{});
+    else
+        march(Flag<false>{});
 }
 
 }  // namespace
@@ -410,19 +448,37 @@ void temporal_box(unsigned* cols, unsigned* rows) {
     *rows = TT_WZ;
 }
 
-cudaError_t launch_temporal_reg(const float* u0, const float* u1, float* v0, float* v1, float wavespeed, float dt,
-                                float dx, float dy, int N, int M, int Mp, bool exact, cudaStream_t s) {
-    constexpr int OZ = TR_H - 2 * TR_HALO;
-    const dim3 grid((M + TR_OX - 1) / TR_OX, (N + OZ - 1) / OZ);
-    const float k = kcoef(wavespeed, dt), dx2 = dx * dx, dy2 = dy * dy;
-    // a plain launch: the window's read-only loads of u0 and u1, the previous
-    // launch's output, are ordered after it by the kernel boundary
-    if (exact)
-        temporal_reg_kernel<true, TR_H, TR_MINB><<<grid, TR_W, 0, s>>>(u0, u1, v0, v1, k, dx2, dy2, k / dx2, k / dy2,
-                                                                     N, M, Mp);
+cudaError_t launch_temporal_stream(const float* u0, const float* u1, float* v0, float* v1, float wavespeed, float dt,
+                                   float dx, float dy, int N, int M, int Mp, cudaStream_t s) {
+    const int strips = (M + TS_COLS - 1) / TS_COLS;
+    // Rows per warp. A warp spends 16 rows on its first and last results. A row takes it
+    // 0.33 us alone and 0.045 more for each warp of its SM, up to the 12 that are resident;
+    // beyond them, more and shorter strips even out the SMs. Measured with S folded into Q,
+    // us: 256^2 8 rows 14.3, 16 rows 18.4; 2048^2 32 rows 35, 20 rows 39, 64 rows 43;
+    // 8000 x 16000 167 rows 425, 250 rows 441, 471 rows 543, 1000 rows 676.
+    int rows = N;
+    double least = 0;
+    for (int q = 1; q <= 64; ++q) {
+        const int n = std::max(1, std::min(304 * q / strips, (N + 3) / 4));
+        const int r = (N + n - 1) / n;
+        const double warps = double(strips) * ((N + r - 1) / r);
+        const double row = warps <= 1824 ? 0.33 + 0.045 * warps / 152 : 0.53 * (warps / 1824 + 0.63);
+        const double cost = row * (r + 16);
+        if (least == 0 || cost < least) {
+            least = cost;
+            rows = r;
+        }
+    }
+    const long long warps = (long long)strips * ((N + rows - 1) / rows);
+    const unsigned ctas = unsigned((warps + TS_WARPS - 1) / TS_WARPS);
+    const float k = kcoef(wavespeed, dt), cx = k / (dx * dx), cy = k / (dy * dy);
+    auto a16 = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    // a plain launch: the copies of u0 and u1, the previous launch's output, are ordered
+    // after it by the kernel boundary
+    if (Mp % 4 == 0 && a16(u0) && a16(u1) && a16(v0) && a16(v1))
+        temporal_stream_kernel<true><<<ctas, 32 * TS_WARPS, 0, s>>>(u0, u1, v0, v1, cx, cy, N, M, Mp, strips, rows);
     else
-        temporal_reg_kernel<false, TR_H, TR_MINB><<<grid, TR_W, 0, s>>>(u0, u1, v0, v1, k, dx2, dy2, k / dx2, k / dy2,
-                                                                      N, M, Mp);
+        temporal_stream_kernel<false><<<ctas, 32 * TS_WARPS, 0, s>>>(u0, u1, v0, v1, cx, cy, N, M, Mp, strips, rows);
     count_launch();
     return cudaGetLastError();
 }

@@ -100,6 +100,9 @@ class BatchFWI:
         self.graph = None  # the library's batch plan (its graph), when graph=True
         self.graph_kernels = 0  # kernels of one replay
         if not graph:
+            for m in self.models:  # side by side: the streaming kernels, as the library's plan does
+                if len(self.models) > 1 and m.call.problem.ndim == 2 and m.call.problem.tile_rows == 0:
+                    m.call.problem.tile_rows = 32
             self._launch()  # eager run: validates arguments
             torch.cuda.synchronize(self.device)
             return

@@ -307,28 +307,31 @@ int check_problem(const wfd_problem* p) {
 // Whether the resident kernel runs the problem, and its splits: the 2D
 // constant-density path with FP32 fields, on grids that fit the chip (for a
 // gradient also with the adjoint's gradient sum in registers), where its estimate
-// is below the streaming kernels' time. Those take about 4 us a step at least and
-// 2 us plus 0.4 M cells per us otherwise (0.44 M for a gradient with two steps per
-// launch, whose recompute overlaps the adjoint). Measured, streaming / resident:
-// forward 256^2 4.1 / 2.2 us, 1024^2 5.7 / 4.1, 2048^2 11.1 / 7.5, 24 shots of
-// 401 x 1203 34 / 22; gradient per step, recompute included, 4 shots of 187 x 243
-// 11.7 / 8.2, 32 shots of 1024^2 with segments of 10 steps 222 / 270 (streamed).
+// is below the streaming kernels' time. A forward streams in about 4 us a step at least
+// and 2 us plus 0.4 M cells per us otherwise. Measured, us a step, streaming / resident:
+// forward 256^2 4.1 / 2.0, 1024^2 5.7 / 4.1, 2048^2 11.1 / 6.7, 24 shots of 401 x 1203
+// 34 / 20; gradient (recompute included) 4 shots of 187 x 243 11.7 / 8.2, 4 shots of
+// 1024^2 41.6 / 30.0, 8 shots 72 / 61, 16 shots 118 / 118, 32 shots 211 / 230 (streamed).
 bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
     if (p->ndim != 2 || p->field_format != WFD_FIELD_FP32 || p->lap_store != WFD_LAP_AUTO ||
         p->adjoint_mode != WFD_ADJOINT_CHECKPOINT || p->level_format != WFD_LEVEL_FP32 || p->step_block > 2 ||
         p->tile_rows > 0 || p->shots_per_cta > 0)  // (a streaming tiling asked for)
         return false;
     const double cells = (double)p->nshot * p->nz * p->nx;
-    const double streamed = std::max(4.0, 2.0 + cells / (grad && p->step_block == 2 ? 440e3 : 400e3));
     const int R = p->order / 2;
     if (!plan_resident(p->nz, p->nx, R, p->nshot, RES_LEAP, f)) return false;
-    if (!grad) return f->step_us < 0.95 * streamed;
+    if (!grad) return f->step_us < 0.95 * std::max(4.0, 2.0 + cells / 400e3);
     if (!plan_resident(p->nz, p->nx, R, p->nshot, RES_ADJOINT, a)) return false;
-    // a gradient: a forward, an adjoint and about one recompute or less, each launch
-    // of a segment with about 12 us of its own (state and m in and out)
+    // A gradient: a forward, an adjoint and a recompute of part of the steps, each launch of
+    // a segment with 4 us of its own and the state and m in and out (8 us for a full chip);
+    // this estimate falls about 14% short. The streaming kernels take 3.2 us per M cells and
+    // step on small batches and 2.2 on large ones, 4 us at least.
     const double seg = p->ckpt_every > 0 ? std::min(p->ckpt_every, p->nt) : std::max(1.0, std::sqrt((double)p->nt));
-    const double fwd = f->step_us + f->passes * 12.0 / seg, adj = a->step_us + a->passes * 12.0 / seg;
-    return 1.6 * fwd + adj < 0.95 * 2.6 * streamed;
+    const double shot = (double)p->nz * p->nx;
+    auto own = [&](const ResPlan& q) { return q.passes * (4.0 + 2e-6 * q.shots * shot) / seg; };
+    const double resident = 1.14 * (1.6 * (f->step_us + own(*f)) + a->step_us + own(*a));
+    const double streamed = std::max(4.0, std::min(3.0 + cells * 3.2e-6, 10.0 + cells * 2.2e-6));
+    return resident < 2.6 * streamed;
 }
 
 // tile_rows > 0 overrides the problem's 2D tile height (3D: the planes per CTA) and step_block >= 1

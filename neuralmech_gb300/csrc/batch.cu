@@ -86,6 +86,11 @@ int wfd_batch_plan(const wfd_batch_item* items, int count, void* stream, wfd_bat
     b->problems.resize(count);
     for (int i = 0; i < count; ++i) {
         b->problems[i] = *items[i].problem;
+        // Models side by side share the chip launch by launch, so they take the streaming
+        // kernels (at their default tile height): the resident one wants every SM for a
+        // whole segment and runs one model after the other. Measured, 5 models of 0.4 .. 0.6 M
+        // cells, 240 steps: 6.3 ms streaming, 10.4 resident.
+        if (count > 1 && b->problems[i].ndim == 2 && b->problems[i].tile_rows == 0) b->problems[i].tile_rows = 32;
         b->items[i].problem = &b->problems[i];
     }
     b->streams.assign(count, nullptr);

@@ -13,6 +13,7 @@ The consumer side of the wave path in projects/18_fwi:
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import numpy as np
 import torch
@@ -24,6 +25,11 @@ from .wavefd import Grid, _ptr, _require_cuda, _stream, wave_forward
 def hilbert_kernel(nt: int) -> np.ndarray:
     """Circular-convolution kernel g of the periodic discrete Hilbert
     transform: g = ifft(-i sign(k)), sign 0 at k = 0 and (even nt) at nt/2."""
+    return _hilbert_kernel(int(nt)).copy()
+
+
+@functools.lru_cache(maxsize=16)
+def _hilbert_kernel(nt: int) -> np.ndarray:
     k = np.arange(nt)
     sgn = np.zeros(nt)
     half = nt // 2
@@ -41,7 +47,7 @@ def analytic_signal(traces: torch.Tensor) -> torch.Tensor:
     _require_cuda(traces, "traces")
     x = traces.to(torch.float32).contiguous()
     nt = x.shape[-1]
-    g = torch.from_numpy(hilbert_kernel(nt)).to(x.device)
+    g = torch.from_numpy(_hilbert_kernel(nt)).to(x.device)
     out = torch.empty(x.shape + (2,), dtype=torch.float32, device=x.device)
     _lib.check(_lib.load().wfd_analytic_signal(_ptr(x), x.numel() // nt, nt, _ptr(g), _ptr(out), _stream()),
                "wfd_analytic_signal")

@@ -24,6 +24,7 @@ exponential (Cerjan) sponge profiles; traces[s, n, r] = u_{n+1}(rec[s, r]).
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 from dataclasses import dataclass, field
 
@@ -169,6 +170,11 @@ def stable_dt(spacing, vmax: float, order: int = 8) -> float:
 
 def sponge_profile(n: int, low: int, high: int, strength: float = 0.3) -> np.ndarray:
     """1D exponential sponge factors g[0..n-1] (1 in the interior)."""
+    return _sponge_profile(int(n), int(low), int(high), float(strength)).copy()
+
+
+@functools.lru_cache(maxsize=64)
+def _sponge_profile(n: int, low: int, high: int, strength: float) -> np.ndarray:
     g = np.ones(n, dtype=np.float64)
     for w, idx in ((low, lambda d: w - d), (high, lambda d: n - 1 - (w - d))):
         if w <= 0:
@@ -224,8 +230,21 @@ def _require_cuda(t: torch.Tensor, name: str):
         raise ValueError(f"{name} must be a CUDA tensor (no CPU path)")
 
 
+def _host_positions(pos, nshot: int, ndim: int) -> np.ndarray:
+    """_positions of positions that are on the host, there."""
+    p = np.asarray(pos)
+    if p.ndim == 2:
+        p = np.broadcast_to(p, (nshot,) + p.shape)
+    if p.ndim != 3 or p.shape[0] != nshot or p.shape[2] != ndim:
+        raise ValueError(f"positions must be (n, {ndim}) or ({nshot}, n, {ndim})")
+    out = np.zeros(p.shape[:2] + (3,), np.int32)
+    out[..., 0] = p[..., 0]
+    out[..., 3 - ndim + 1:] = p[..., 1:]
+    return out
+
+
 def _positions(pos, nshot: int, ndim: int, device) -> torch.Tensor:
-    """(nshot, n, 3) int32 (z, y, x) from (n, ndim) or (nshot, n, ndim)."""
+    """(nshot, n, 3) int32 (z, y, x) on the device from (n, ndim) or (nshot, n, ndim)."""
     p = torch.as_tensor(pos, device=device)
     if p.dim() == 2:
         p = p.unsqueeze(0).expand(nshot, -1, -1)
@@ -235,6 +254,23 @@ def _positions(pos, nshot: int, ndim: int, device) -> torch.Tensor:
     if ndim == 2:
         p = torch.stack([p[..., 0], torch.zeros_like(p[..., 0]), p[..., 1]], dim=-1)
     return p.contiguous()
+
+
+def _to_device(arrays, device) -> list:
+    """Device tensors of several small host arrays (None stays None): one copy for
+    all of them, each on a 256-byte boundary of one buffer."""
+    at, n = [], 0
+    for a in arrays:
+        at.append(n)
+        n += 0 if a is None else (a.nbytes + 255) // 256 * 256
+    host = np.empty(n, np.uint8)
+    for a, o in zip(arrays, at):
+        if a is not None:
+            host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)
+    buf = torch.from_numpy(host).to(device)
+    kinds = {np.dtype(np.int32): torch.int32, np.dtype(np.float32): torch.float32}
+    return [None if a is None else buf[o:o + a.nbytes].view(kinds[a.dtype]).view(a.shape)
+            for a, o in zip(arrays, at)]
 
 
 def _wavelet(w, nshot: int, nt: int, nsrc: int, device) -> torch.Tensor:
@@ -266,17 +302,22 @@ def _prepare(vel, wavelet, src, rec, grid: Grid, nshot=None) -> _Call:
         raise ValueError(f"vel has shape {tuple(vel.shape)}, grid {grid.shape}")
     vel = vel.detach().to(torch.float32).contiguous()
     dev = vel.device
-    src_t = torch.as_tensor(src)
     if nshot is None:
-        nshot = src_t.shape[0] if src_t.dim() == 3 else 1
-    srcp = _positions(src, nshot, grid.ndim, dev)
-    recp = _positions(rec, nshot, grid.ndim, dev)
+        shape = np.shape(src)
+        nshot = shape[0] if len(shape) == 3 else 1
+    # positions on the host travel with the sponge factors, in one copy
+    on_host = [not (isinstance(p, torch.Tensor) and p.is_cuda) for p in (src, rec)]
+    sp = sponge_profiles(grid)
+    host = [_host_positions(p, nshot, grid.ndim) if h else None for p, h in zip((src, rec), on_host)]
+    srcp, recp, *sp = _to_device([*host, *sp], dev)
+    if not on_host[0]:
+        srcp = _positions(src, nshot, grid.ndim, dev)
+    if not on_host[1]:
+        recp = _positions(rec, nshot, grid.ndim, dev)
     wav = _wavelet(wavelet, nshot, grid.nt, srcp.shape[1], dev)
     vmax = float(vel.max())
     prob = _problem(grid, nshot, srcp.shape[1], recp.shape[1], vmax)
-    gz, gy, gx = sponge_profiles(grid)
-    sp = tuple(None if g is None else torch.from_numpy(g).to(dev) for g in (gz, gy, gx))
-    return _Call(grid, prob, vel, wav, srcp, recp, sp)
+    return _Call(grid, prob, vel, wav, srcp, recp, tuple(sp))
 
 
 def workspace_bytes(grid: Grid, nshot: int, nsrc: int, nrec: int, with_gradient: bool) -> int:

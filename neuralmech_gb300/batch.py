@@ -101,8 +101,9 @@ class BatchFWI:
         self.graph_kernels = 0  # kernels of one replay
         if not graph:
             for m in self.models:  # side by side: the streaming kernels, as the library's plan does
-                if len(self.models) > 1 and m.call.problem.ndim == 2 and m.call.problem.tile_rows == 0:
-                    m.call.problem.tile_rows = 32
+                p = m.call.problem
+                if len(self.models) > 1 and p.ndim == 2 and p.tile_rows == 0 and p.shots_per_cta == 0:
+                    p.tile_rows = 32
             self._launch()  # eager run: validates arguments
             torch.cuda.synchronize(self.device)
             return

@@ -304,6 +304,34 @@ int check_problem(const wfd_problem* p) {
     return WFD_OK;
 }
 
+}  // namespace
+
+// Shots per CTA of a streaming kernel. In units of one shot's tile, a CTA costs its shots
+// plus 0.55 (barriers, m, the sponge and its first, unhidden loads), and the launch ends
+// in about 0.45 of a CTA's time during which the chip empties; `share` is how many
+// times this work runs beside it (the other models of a batch). Measured, us: gradient of
+// 12 shots of 480 x 760, variable density, 240 steps, 1 / 2 / 3 / 4 / 6 shots per CTA
+// 23014 / 21620 / 20772 / 20891 / 24250; of 32 shots of 1024^2, 1 / 2 / 4 / 8 / 16 / 32 119.9 /
+// 96.6 / 86.9 / 84.1 / 84.5 / 93.0 ms; 4 models of 5 shots side by side, 1 / 2 / 3 / 5 12.9 /
+// 11.2 / 10.4 / 10.5 ms.
+int wfd::auto_spc(int ntiles, int nshot, double share) {
+    int best = 1;
+    double least = 0;
+    for (int s = 1; s <= std::min(nshot, T2_MAX_SPC); ++s) {
+        const long long groups = (nshot + s - 1) / s;
+        if (groups > 65535) continue;  // (gridDim.y)
+        const double work = share * ntiles * (nshot + 0.55 * groups) / 304.0;  // 2 CTAs on 152 SMs
+        const double t = std::max(work, s + 0.55) + 0.45 * (s + 0.55);
+        if (least == 0 || t < least) {
+            least = t;
+            best = s;
+        }
+    }
+    return best;
+}
+
+namespace {
+
 // Whether the resident kernel runs the problem, and its splits: the 2D
 // constant-density path with FP32 fields, on grids that fit the chip (for a
 // gradient also with the adjoint's gradient sum in registers), where its estimate
@@ -394,13 +422,7 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
     } else if (p->shots_per_cta > 0) {
         g.spc = std::min(std::min(p->shots_per_cta, p->nshot), T2_MAX_SPC);
     } else {
-        // enough CTAs for ~6 waves of 2 resident CTAs on 152 SMs, otherwise
-        // as many shots per CTA as possible (m and the gradient amortise over them)
-        const long long target = 152LL * 2 * 6;
-        long long spc = (long long)g.ntiles * p->nshot / target;
-        int s = 1;
-        while (2LL * s <= spc && 2 * s <= p->nshot) s *= 2;
-        g.spc = std::min(s, T2_MAX_SPC);
+        g.spc = auto_spc(g.ntiles, p->nshot, 1.0);
     }
     // (the shot count is bounded so that nshot / T2_MAX_SPC CTA rows fit gridDim.y)
     g.K = p->ckpt_every > 0 ? std::min(p->ckpt_every, p->nt)

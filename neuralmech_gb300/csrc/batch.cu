@@ -10,6 +10,7 @@
 // (projects/18_simple_wave_fd/2D_wave_cuda_graph.py:73-95, a captured
 // sequence of padded_step launches replayed per block of steps), for whole
 // gradients of several models.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <new>
@@ -86,12 +87,21 @@ int wfd_batch_plan(const wfd_batch_item* items, int count, void* stream, wfd_bat
     b->problems.resize(count);
     for (int i = 0; i < count; ++i) {
         b->problems[i] = *items[i].problem;
-        // Models side by side share the chip launch by launch, so they take the streaming
-        // kernels (at their default tile height): the resident one wants every SM for a
-        // whole segment and runs one model after the other. Measured, 5 models of 0.4 .. 0.6 M
-        // cells, 240 steps: 6.3 ms streaming, 10.4 resident.
-        if (count > 1 && b->problems[i].ndim == 2 && b->problems[i].tile_rows == 0) b->problems[i].tile_rows = 32;
         b->items[i].problem = &b->problems[i];
+    }
+    // Models side by side share the chip launch by launch. So they take the streaming
+    // kernels, with shots per CTA for the whole batch's work: the resident kernel wants
+    // every SM for a segment and would run one model after the other. Measured, 5 models of
+    // 0.4 .. 0.6 M cells, 240 steps: 6.3 ms streaming, 10.4 resident.
+    if (count > 1) {
+        double all = 0;
+        for (const wfd_problem& p : b->problems) all += (double)p.nshot * p.nz * p.nx;
+        for (wfd_problem& p : b->problems) {
+            if (p.ndim != 2 || p.shots_per_cta != 0 || p.tile_rows != 0 || p.step_block > 2) continue;
+            // (tiles of 3 K cells: between the two-step kernel's 120 x 24 and the others')
+            const double cells = (double)p.nz * p.nx;
+            p.shots_per_cta = wfd::auto_spc(std::max(1, int(cells / 3000)), p.nshot, all / (cells * p.nshot));
+        }
     }
     b->streams.assign(count, nullptr);
     b->joins.assign(count, nullptr);

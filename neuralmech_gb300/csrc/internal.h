@@ -315,6 +315,9 @@ void count_launch(int n = 1);
 // Records `message` as the calling thread's wfd_last_error() and returns status.
 int set_error(int status, const char* message);
 
+// Shots per CTA of a streaming 2D kernel (api.cu).
+int auto_spc(int ntiles, int nshot, double share);
+
 // ---------------------------------------------------------------- helpers (aux.cu)
 cudaError_t launch_vel_to_m(const float* vel, float* m, int nz, int ny, int nx, int ld,
                             float scale, cudaStream_t s);

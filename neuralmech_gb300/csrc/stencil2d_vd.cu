@@ -179,17 +179,45 @@ __global__ void __launch_bounds__(VD_THREADS, 2)
     auto fluxes = [&](const float* T, float4* dxr, float4* dzr) {
         auto trow = [&](int fr) { return T + fr * VD_W; };  // staged row of z = z0 - 2R + fr
         auto brow = [&](int br) { return B + br * VD_W; };  // staged b row of z = z0 - R + br
+        // z: own half rows zb, zb + 1 from a window of field rows zb - R + 1 .. zb + R; the
+        // window's rows zb, zb + 1 and the b rows serve the x fluxes too (28 instead of 33
+        // row loads a field from shared memory, whose pipe is 62% busy: 20.42 -> 20.20 ms)
+        float4 bb[VD_RB + 1];
+#pragma unroll
+        for (int r = 0; r <= VD_RB; ++r) bb[r] = ld4(brow(warp * VD_RB + r + R) + 8 + 4 * lane);
+        float4 own[VD_RB];
+        {
+            float4 W[VD_RB + 2 * R - 1];
+#pragma unroll
+            for (int j = 0; j < VD_RB + 2 * R - 1; ++j) W[j] = ld4(trow(warp * VD_RB + R + 1 + j) + 8 + 4 * lane);
+#pragma unroll
+            for (int r = 0; r < VD_RB; ++r) {
+                own[r] = W[R - 1 + r];
+                float2 dl = make_float2(0.f, 0.f), dh = dl;
+#pragma unroll
+                for (int k = 1; k <= R; ++k) {
+                    const float4 up = W[r + R - 1 + k], dn = W[r + R - k];
+                    dl = __ffma2_rn(a.csp[k - 1], psub(lo2v(up), lo2v(dn)), dl);
+                    dh = __ffma2_rn(a.csp[k - 1], psub(hi2v(up), hi2v(dn)), dh);
+                }
+                dzr[r] = make_float4(dl.x, dl.y, dh.x, dh.y);
+                const float2 h = make_float2(0.5f, 0.5f);
+                const float2 fl = __fmul2_rn(__fmul2_rn(h, __fadd2_rn(lo2v(bb[r]), lo2v(bb[r + 1]))), dl);
+                const float2 fh = __fmul2_rn(__fmul2_rn(h, __fadd2_rn(hi2v(bb[r]), hi2v(bb[r + 1]))), dh);
+                st4(FZ + (warp * VD_RB + r + R) * VD_TX + 4 * lane, make_float4(fl.x, fl.y, fh.x, fh.y));
+            }
+        }
         // x: own half points x .. x + 3 of the rows zb, zb + 1
 #pragma unroll
         for (int r = 0; r < VD_RB; ++r) {
             const int fr = warp * VD_RB + r + 2 * R, br = warp * VD_RB + r + R;
-            const float4 p0 = ld4(trow(fr) + 4 * lane + 4), p1 = ld4(trow(fr) + 4 * lane + 8),
-                         p2 = ld4(trow(fr) + 4 * lane + 12);
+            const float4 p0 = ld4(trow(fr) + 4 * lane + 4), p1 = own[r], p2 = ld4(trow(fr) + 4 * lane + 12);
             const float w[12] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w, p2.x, p2.y, p2.z, p2.w};
             const float4 d = dx4<R>(w, a);
-            const float4 b0 = ld4(brow(br) + 4 * lane + 8), b1 = ld4(brow(br) + 4 * lane + 12);
+            const float4 b0 = bb[r];
+            const float b1 = brow(br)[4 * lane + 12];
             const float4 bx = make_float4(0.5f * (b0.x + b0.y), 0.5f * (b0.y + b0.z), 0.5f * (b0.z + b0.w),
-                                          0.5f * (b0.w + b1.x));
+                                          0.5f * (b0.w + b1));
             dxr[r] = d;
             st4(FX + (warp * VD_RB + r) * VD_FXW + 4 + 4 * lane,
                 make_float4(bx.x * d.x, bx.y * d.y, bx.z * d.z, bx.w * d.w));
@@ -208,29 +236,6 @@ __global__ void __launch_bounds__(VD_THREADS, 2)
             for (int k = 1; k <= R; ++k) d = fmaf(a.cs[k - 1], tr[sc + k] - tr[sc - k + 1], d);
             const float bx = 0.5f * (brow(br)[sc] + brow(br)[sc + 1]);
             FX[(warp * VD_RB + r) * VD_FXW + (h < 4 ? h : VD_TX + h)] = bx * d;
-        }
-        // z: own half rows zb, zb + 1 from a window of field rows zb - R + 1 .. zb + R
-        {
-            float4 W[VD_RB + 2 * R - 1];
-#pragma unroll
-            for (int j = 0; j < VD_RB + 2 * R - 1; ++j) W[j] = ld4(trow(warp * VD_RB + R + 1 + j) + 8 + 4 * lane);
-#pragma unroll
-            for (int r = 0; r < VD_RB; ++r) {
-                float2 dl = make_float2(0.f, 0.f), dh = dl;
-#pragma unroll
-                for (int k = 1; k <= R; ++k) {
-                    const float4 up = W[r + R - 1 + k], dn = W[r + R - k];
-                    dl = __ffma2_rn(a.csp[k - 1], psub(lo2v(up), lo2v(dn)), dl);
-                    dh = __ffma2_rn(a.csp[k - 1], psub(hi2v(up), hi2v(dn)), dh);
-                }
-                const int br = warp * VD_RB + r + R;
-                const float4 b0 = ld4(brow(br) + 8 + 4 * lane), b1 = ld4(brow(br + 1) + 8 + 4 * lane);
-                dzr[r] = make_float4(dl.x, dl.y, dh.x, dh.y);
-                const float2 h = make_float2(0.5f, 0.5f);
-                const float2 fl = __fmul2_rn(__fmul2_rn(h, __fadd2_rn(lo2v(b0), lo2v(b1))), dl);
-                const float2 fh = __fmul2_rn(__fmul2_rn(h, __fadd2_rn(hi2v(b0), hi2v(b1))), dh);
-                st4(FZ + (warp * VD_RB + r + R) * VD_TX + 4 * lane, make_float4(fl.x, fl.y, fh.x, fh.y));
-            }
         }
         // z halo half rows: FZ rows 0 .. R-1 (warps 0 .. R-1) and VD_TZ + R .. VD_TZ + 2R - 2
         if (warp < 2 * R - 1) {
@@ -302,6 +307,19 @@ __global__ void __launch_bounds__(VD_THREADS, 2)
             }
         }
         float4 dxq[VD_RB], dzq[VD_RB], lb[VD_RB];
+        // MODE_GRAD_U: u_{n-1} comes from global memory (plain loads: u_new is
+        // this level's buffer, each cell read here and written below); issued
+        // before the fluxes so that their latency overlaps both sums (between the
+        // fluxes and the divergence: 46 us a launch at 12 shots of 480 x 760, 3 of 9
+        // stall cycles on loads; the gradient there 20.74 -> 20.42 ms)
+        float4 ovg[MODE == MODE_GRAD_U ? VD_RB : 1];
+        if (MODE == MODE_GRAD_U) {
+#pragma unroll
+            for (int r = 0; r < VD_RB; ++r)
+                ovg[r] = (zb + r < a.nz && x < a.ld)
+                             ? *reinterpret_cast<const float4*>(un + (long long)(zb + r) * a.ld + x)
+                             : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
         fluxes(F, dxq, dzq);
         if (MODE == MODE_GRAD_U) {  // the half-point terms now: the four differences die here
 #pragma unroll
@@ -317,17 +335,6 @@ __global__ void __launch_bounds__(VD_THREADS, 2)
             }
         }
         __syncthreads();
-        // MODE_GRAD_U: u_{n-1} comes from global memory (plain loads: u_new is
-        // this level's buffer, each cell read here and written below); issued
-        // before the divergence so that their latency overlaps it
-        float4 ovg[MODE == MODE_GRAD_U ? VD_RB : 1];
-        if (MODE == MODE_GRAD_U) {
-#pragma unroll
-            for (int r = 0; r < VD_RB; ++r)
-                ovg[r] = (zb + r < a.nz && x < a.ld)
-                             ? *reinterpret_cast<const float4*>(un + (long long)(zb + r) * a.ld + x)
-                             : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
         divergence(lb);
 
 #pragma unroll

@@ -362,11 +362,12 @@ bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
     return resident < 2.6 * streamed;
 }
 
-// tile_rows > 0 overrides the problem's 2D tile height (3D: the planes per CTA) and step_block >= 1
+// tile_rows > 0 overrides the problem's 2D tile height (3D: the planes per CTA, on
+// columns column_x wide) and step_block >= 1
 // its steps per launch (the u-store adjoint runs one step per launch on
 // 16-row tiles: its third staged tile must leave room for the stages).
 Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool vd = false,
-               const ResPlan* rf = nullptr, const ResPlan* ra = nullptr) {
+               const ResPlan* rf = nullptr, const ResPlan* ra = nullptr, int column_x = T3_TX) {
     Geom g{};
     if (rf) {
         g.res = true;
@@ -410,8 +411,10 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
         g.tile_y = 1;
         g.tile_x = T2_TX;
     } else {
-        g.tile_z = tile_rows > 0 ? tile_rows : plan_zchunk3d(g.nz, g.ny, g.nx, p->nshot);
-        g.tile_y = T3_TY; g.tile_x = T3_TX;
+        g.tile_z = tile_rows;
+        g.tile_x = column_x;
+        if (tile_rows <= 0) plan_columns3d(g.nz, g.ny, g.nx, p->nshot, &g.tile_x, &g.tile_z);
+        g.tile_y = T3_CELLS / g.tile_x;
     }
     g.tiles_z = cdiv(g.nz, g.tile_z);
     g.tiles_y = cdiv(g.ny, g.tile_y);
@@ -687,7 +690,7 @@ Geom call_geom(const wfd_problem* p, bool grad, size_t workspace_bytes) {
 
 // The geometry of a later shot group, which may be smaller than the first (gf).
 Geom group_geom(const wfd_problem* q, const Geom& gf) {
-    if (gf.ndim == 3) return make_geom(q, gf.tile_z);
+    if (gf.ndim == 3) return make_geom(q, gf.tile_z, 0, false, nullptr, nullptr, gf.tile_x);
     return gf.res ? make_geom(q, 0, 0, false, &gf.rf, gf.ra.rb > 0 ? &gf.ra : nullptr) : make_geom(q);
 }
 
@@ -736,7 +739,7 @@ struct Stepper {
         if (!enc) return fail(WFD_ERR_CUDA, "cuTensorMapEncodeTiled entry point unavailable");
         const cuuint64_t dims[3] = {(cuuint64_t)g.nx, (cuuint64_t)g.ny, (cuuint64_t)g.nz};
         const cuuint64_t strides[2] = {(cuuint64_t)g.ld * 4, (cuuint64_t)g.plane * 4};
-        const cuuint32_t box[3] = {T3_TX, T3_TY, 1}, estr[3] = {1, 1, 1};
+        const cuuint32_t box[3] = {cuuint32_t(g.tile_x), cuuint32_t(g.tile_y), 1}, estr[3] = {1, 1, 1};
         CUresult r = enc(&map_m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(m), dims,
                          strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -759,6 +762,7 @@ struct Stepper {
         a.shots_per_cta = g.spc;
         a.tiles_x = g.tiles_x; a.tiles_y = g.tiles_y; a.tiles_z = g.tiles_z;
         a.tile_z = g.tile_z;
+        a.tile_x = g.tile_x;
         a.c0 = g.c0;
         for (int k = 0; k < 4; ++k) { a.cz[k] = g.cz[k]; a.cy[k] = g.cy[k]; a.cx[k] = g.cx[k]; }
         a.zero_ring = 1;  // the wave path's ring is 0 in every level
@@ -784,8 +788,8 @@ struct Stepper {
             if ((rc = make_field_map(mc, cur, false, 2, g.nz, 1, g.nx, g.ld, p->nshot, bc))) return rc;
             return make_field_map(mo, old, false, 2, g.nz, 1, g.nx, g.ld, p->nshot, bo);
         }
-        const cuuint32_t bc[4] = {T3_W, cuuint32_t(T3_TY + 2 * g.R), 1, 1};
-        const cuuint32_t bo[4] = {T3_TX, T3_TY, 1, 1};
+        const cuuint32_t bc[4] = {cuuint32_t(g.tile_x + 2 * T3_XH), cuuint32_t(g.tile_y + 2 * g.R), 1, 1};
+        const cuuint32_t bo[4] = {cuuint32_t(g.tile_x), cuuint32_t(g.tile_y), 1, 1};
         if ((rc = make_field_map(mc, cur, false, 3, g.nz, g.ny, g.nx, g.ld, p->nshot, bc))) return rc;
         return make_field_map(mo, old, false, 3, g.nz, g.ny, g.nx, g.ld, p->nshot, bo);
     }
@@ -795,7 +799,7 @@ struct Stepper {
             const cuuint32_t b[3] = {T2_TX, cuuint32_t(g.tile_z), 1};
             return make_field_map(ml, lap, bf16, 2, g.nz, 1, g.nx, g.ld, p->nshot, b);
         }
-        const cuuint32_t b[4] = {T3_TX, T3_TY, 1, 1};
+        const cuuint32_t b[4] = {cuuint32_t(g.tile_x), cuuint32_t(g.tile_y), 1, 1};
         return make_field_map(ml, lap, bf16, 3, g.nz, g.ny, g.nx, g.ld, p->nshot, b);
     }
 

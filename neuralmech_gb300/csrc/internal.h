@@ -8,7 +8,7 @@ namespace wfd {
 
 // Device error bits, OR-ed into the workspace's status word.
 enum : unsigned {
-    DEV_ERR_TMA_TIMEOUT = 1u << 0,   // an mbarrier wait for a TMA tile gave up
+    DEV_ERR_TMA_TIMEOUT = 1u << 0,   // a wait for a TMA tile or a neighbour's halo gave up
     DEV_ERR_BAD_POSITION = 1u << 1,  // a source/receiver outside the updated interior
 };
 
@@ -67,7 +67,7 @@ struct StepArgs {
     long long shot_stride;     // cells per shot (nz * plane)
     int nshot, shots_per_cta;
     int tiles_x, tiles_y, tiles_z;
-    int tile_z;                // 3D: output planes per CTA (at most T3_ZCHUNK)
+    int tile_z, tile_x;        // 3D: output planes per CTA (at most T3_ZCHUNK), width of its column
     float c0;                  // centre weight (all axes)
     float cz[4], cy[4], cx[4]; // axis weights for k = 1..R, already scaled by (dx/h)^2
     float2 c0p, czp[4], cyp[4], cxp[4]; // the same as duplicated pairs, operands of the
@@ -286,24 +286,29 @@ cudaError_t launch_wave_reg(int R, const StepArgs& a, const RegArgs& q, cudaStre
 // One CTA (one shot) marches along z through a (TY x TX) column of the grid
 // for T3_ZCHUNK output planes; a thread owns 4 x cells and keeps the 2R + 1
 // z taps of each in registers.
-constexpr int T3_TX = 64;
+constexpr int T3_TX = 64;                        // the two column shapes: 64 x 16 ...
 constexpr int T3_TY = 16;
+constexpr int T3_TX2 = 32;                       // ... and 32 x 32 cells
+constexpr int T3_CELLS = T3_TX * T3_TY;
 constexpr int T3_XH = 4;
-constexpr int T3_W = T3_TX + 2 * T3_XH;
 constexpr int T3_ROWS = 1;                       // tile rows per thread
-constexpr int T3_THREADS = (T3_TX / 4) * T3_TY / T3_ROWS;
+constexpr int T3_THREADS = T3_CELLS / 4 / T3_ROWS;
 constexpr int T3_ZCHUNK = 64;                    // planes per CTA at most (z blocking)
 
-// Planes per CTA. A CTA spends about 6 planes' time on filling its queues and rings,
+// Shape of a column and planes per CTA. A CTA spends about 6 planes' time on filling its queues and rings,
 // so a large grid takes T3_ZCHUNK; a small one takes what fills the chip's two CTAs
 // per SM with the fewest planes in a row. Measured, us a step at 64 planes / planned:
 // 64^3 98 / 20 (8 planes), 2 shots of 97 x 131 x 149 50 / 24 (20), 160^3 51 / 21 (8),
 // gradient of 4 shots of 144 x 128 x 160 68 / 52 per launch (48).
-int plan_zchunk3d(int nz, int ny, int nx, int nshot);
+// The shape is the one that covers the grid with the less work (32 x 32 cells have 7%
+// less halo to stage, which is not what bounds the kernel: ties keep 64 x 16). us a step,
+// 64 x 16 / 32 x 32: 2 shots of 97 x 131 x 149 24 / 21, of 120 x 150 x 90 26 / 20, 160^3
+// 23 / 21; 256^3, where both cover it alike, 68 / 68.
+void plan_columns3d(int nz, int ny, int nx, int nshot, int* tile_x, int* planes);
 
-// map_cur: u_n planes (box T3_W x (T3_TY + 2R) x 1 x 1); map_old, map_lap:
-// output-plane tiles (box T3_TX x T3_TY x 1 x 1); map_m: the model m
-// ([z][y][ld], box T3_TX x T3_TY x 1).
+// map_cur: u_n planes (box (TX + 2 T3_XH) x (TY + 2R) x 1 x 1, TX = a.tile_x, TY =
+// T3_CELLS / TX); map_old, map_lap: output-plane tiles (box TX x TY x 1 x 1); map_m: the
+// model m ([z][y][ld], box TX x TY x 1).
 cudaError_t launch_step3d(int R, int mode, const CUtensorMap& map_cur, const CUtensorMap& map_old,
                           const CUtensorMap& map_lap, const CUtensorMap& map_m, const StepArgs& a,
                           cudaStream_t s);

@@ -4,9 +4,9 @@
 //   u_{n+1} = g (2 u_n + m L u_n) - g^2 u_{n-1},  g = gz[z] gy[y] gx[x],
 // on fields [shot][z][y][ld] FP32 (x fastest, ld a multiple of 8).
 //
-// Per CTA (256 threads = 16 lanes along x x 16 rows along y): one shot, one
-// 64 x 16 (x, y) column, marching along z through a.tile_z output planes (at most
-// T3_ZCHUNK; fewer on small grids, chosen by plan_zchunk3d).
+// Per CTA (256 threads, each 4 cells of a row): one shot, one (x, y) column of 64 x 16
+// or 32 x 32 cells (a.tile_x), marching along z through a.tile_z output planes (at most
+// T3_ZCHUNK; fewer on small grids; plan_columns3d chooses both).
 // The shot is the fastest grid index: the CTAs of all shots of one column run
 // together, so m and (MODE_GRAD) the gradient tile are read from DRAM once
 // per column and served from L2 to the other shots.
@@ -38,15 +38,16 @@ namespace {
 __host__ __device__ constexpr int align3(int v, int a) { return (v + a - 1) / a * a; }
 
 constexpr int NBO = 4;  // u_{n-1} / m / L u tile ring (the u_n ring has NBO + R buffers)
-constexpr int LANES_X = T3_TX / 4;  // 16
 
-template <int R, int MODE>
+template <int R, int MODE, int TX>
 struct Layout3D {
+    static constexpr int TY = T3_CELLS / TX;  // rows of a column
+    static constexpr int W = TX + 2 * T3_XH;  // staged columns
     static constexpr int NB = NBO + R;  // u_n plane ring
-    static constexpr int H = T3_TY + 2 * R;
-    static constexpr int CUR = H * T3_W * 4;  // TMA box bytes of one u_n plane
+    static constexpr int H = TY + 2 * R;
+    static constexpr int CUR = H * W * 4;  // TMA box bytes of one u_n plane
     static constexpr int CUR_AL = align3(CUR, 128);
-    static constexpr int TILE = T3_TY * T3_TX * 4;  // one FP32 output-plane tile
+    static constexpr int TILE = TY * TX * 4;  // one FP32 output-plane tile
     static constexpr int OLD_GROUP = 2 * TILE + (MODE == MODE_GRAD ? TILE : 0);  // old, m, lap
     static constexpr int BYTES = NB * CUR_AL + NBO * OLD_GROUP + NB * 8 + T3_ZCHUNK * 4 + 128;
 };
@@ -54,16 +55,16 @@ struct Layout3D {
 __device__ __forceinline__ float2 lo2(const float4& v) { return make_float2(v.x, v.y); }
 __device__ __forceinline__ float2 hi2(const float4& v) { return make_float2(v.z, v.w); }
 
-template <int R, int MODE, int TR>
-__global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
+template <int R, int MODE, int TR, int TX>
+__global__ void __launch_bounds__(T3_THREADS, 2)
     step3d_kernel(const __grid_constant__ CUtensorMap map_cur,
                   const __grid_constant__ CUtensorMap map_old,
                   const __grid_constant__ CUtensorMap map_lap,
                   const __grid_constant__ CUtensorMap map_m, const StepArgs a) {
-    using L = Layout3D<R, MODE>;
-    constexpr int NB = L::NB;
+    using L = Layout3D<R, MODE, TX>;
+    constexpr int NB = L::NB, TY = L::TY, W = L::W, LANES_X = TX / 4;
     constexpr int Q = 2 * R + 1;                 // z taps held in registers per row
-    constexpr int NTH = LANES_X * T3_TY / TR;    // threads
+    constexpr int NTH = LANES_X * TY / TR;       // threads
     constexpr int YW = TR + 2 * R;               // staged rows a thread reads for its y taps
     extern __shared__ unsigned char smem_raw[];
     unsigned char* base = reinterpret_cast<unsigned char*>(
@@ -81,11 +82,11 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
     const int tx_i = tile % a.tiles_x;
     const int ty_i = (tile / a.tiles_x) % a.tiles_y;
     const int tz_i = tile / (a.tiles_x * a.tiles_y);
-    const int x0 = tx_i * T3_TX, y0 = ty_i * T3_TY, z0 = tz_i * a.tile_z;
+    const int x0 = tx_i * TX, y0 = ty_i * TY, z0 = tz_i * a.tile_z;
     const int zc = min(a.tile_z, a.nz - z0);  // output planes of this CTA
     const int total = zc + 2 * R;               // u_n planes it stages
 
-    const uint32_t lap_bytes = MODE == MODE_GRAD ? uint32_t(T3_TY * T3_TX * (a.lap_bf16 ? 2 : 4)) : 0u;
+    const uint32_t lap_bytes = MODE == MODE_GRAD ? uint32_t(TY * TX * (a.lap_bf16 ? 2 : 4)) : 0u;
     auto cur_buf = [&](int p) { return reinterpret_cast<float*>(cur_ring + (p % NB) * L::CUR_AL); };
     auto old_buf = [&](int zr) { return reinterpret_cast<float*>(old_ring + (zr % NBO) * L::OLD_GROUP); };
     auto m_buf = [&](int zr) { return reinterpret_cast<float*>(old_ring + (zr % NBO) * L::OLD_GROUP + L::TILE); };
@@ -147,7 +148,7 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
         if (!mbar_wait(&bc[p % NB], (p / NB) & 1)) report(a.err, DEV_ERR_TMA_TIMEOUT);
 #pragma unroll
         for (int t = 0; t < TR; ++t)
-            V[t][p + 1] = *reinterpret_cast<const float4*>(cur_buf(p) + (yr0 + t + R) * T3_W + col);
+            V[t][p + 1] = *reinterpret_cast<const float4*>(cur_buf(p) + (yr0 + t + R) * W + col);
     }
     __syncthreads();  // planes 0 .. R-1 are consumed
     if (tid == 0) {
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
         for (int t = 0; t < TR; ++t) {
 #pragma unroll
             for (int j = 0; j < 2 * R; ++j) V[t][j] = V[t][j + 1];
-            V[t][2 * R] = *reinterpret_cast<const float4*>(cur_buf(pn) + (yr0 + t + R) * T3_W + col);
+            V[t][2 * R] = *reinterpret_cast<const float4*>(cur_buf(pn) + (yr0 + t + R) * W + col);
         }
 
         const float* pl = cur_buf(zr + R);  // u_n at the output plane, with halo
@@ -179,13 +180,13 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
             if (j >= R && j < R + TR)
                 Y[j] = V[j - R][R];
             else
-                Y[j] = *reinterpret_cast<const float4*>(pl + (yr0 + j) * T3_W + col);
+                Y[j] = *reinterpret_cast<const float4*>(pl + (yr0 + j) * W + col);
         }
         const float gz = gzs[zr];
         const bool zin = z >= R && z < a.nz - R;
 #pragma unroll
         for (int t = 0; t < TR; ++t) {
-            const float* prow = pl + (yr0 + t + R) * T3_W + 4 * lane;
+            const float* prow = pl + (yr0 + t + R) * W + 4 * lane;
             const float4 lv = *reinterpret_cast<const float4*>(prow);
             const float4 cv = V[t][R];
             const float4 rv = *reinterpret_cast<const float4*>(prow + 2 * T3_XH);
@@ -216,7 +217,7 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
             }
             lo = __fadd2_rn(__fadd2_rn(lo, loy), loz);
             hi = __fadd2_rn(__fadd2_rn(hi, hiy), hiz);
-            const int ti = (yr0 + t) * T3_TX + 4 * lane;
+            const int ti = (yr0 + t) * TX + 4 * lane;
             const float4 ov = *reinterpret_cast<const float4*>(old_buf(zr) + ti);
             const float4 mv = *reinterpret_cast<const float4*>(m_buf(zr) + ti);
             // u_{n+1} = g (m L u + 2 u) - g^2 u_{n-1}
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
             if (pz != z) continue;
             const int rem = en.x - pz * int(a.plane);
             const int py = rem / a.ld, px = rem - py * a.ld;
-            float v = pl[(py - y0 + R) * T3_W + (px - x0 + T3_XH)] * a.smp_scale;
+            float v = pl[(py - y0 + R) * W + (px - x0 + T3_XH)] * a.smp_scale;
             if (a.smp_div_m) v /= a.m[en.x];
             a.smp_out[((long long)s * a.smp_nt + a.smp_t) * a.smp_np + en.y] = v;
         }
@@ -327,24 +328,31 @@ __global__ void __launch_bounds__(LANES_X * T3_TY / TR, 2)
     }
 }
 
-template <int R, int MODE>
-cudaError_t launch_impl(const CUtensorMap& mc, const CUtensorMap& mo, const CUtensorMap& ml,
+template <int R, int MODE, int TX>
+cudaError_t launch_tile(const CUtensorMap& mc, const CUtensorMap& mo, const CUtensorMap& ml,
                         const CUtensorMap& mm, const StepArgs& a, cudaStream_t s) {
-    using L = Layout3D<R, MODE>;
+    using L = Layout3D<R, MODE, TX>;
     static int configured_device = -1;
     int dev = 0;
     cudaGetDevice(&dev);
     if (configured_device != dev) {
-        cudaError_t e = cudaFuncSetAttribute(step3d_kernel<R, MODE, T3_ROWS>,
+        cudaError_t e = cudaFuncSetAttribute(step3d_kernel<R, MODE, T3_ROWS, TX>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES);
         if (e != cudaSuccess) return e;
         configured_device = dev;
     }
     const dim3 grid(a.nshot, a.tiles_x * a.tiles_y * a.tiles_z);
-    const cudaError_t e = launch_pdl(step3d_kernel<R, MODE, T3_ROWS>, grid, dim3(T3_THREADS), L::BYTES, s, mc, mo, ml, mm,
+    const cudaError_t e = launch_pdl(step3d_kernel<R, MODE, T3_ROWS, TX>, grid, dim3(T3_THREADS), L::BYTES, s, mc, mo, ml, mm,
                                      with_weight_pairs(a));
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+
+template <int R, int MODE>
+cudaError_t launch_impl(const CUtensorMap& mc, const CUtensorMap& mo, const CUtensorMap& ml,
+                        const CUtensorMap& mm, const StepArgs& a, cudaStream_t s) {
+    return a.tile_x == T3_TX ? launch_tile<R, MODE, T3_TX>(mc, mo, ml, mm, a, s)
+                             : launch_tile<R, MODE, T3_TX2>(mc, mo, ml, mm, a, s);
 }
 
 template <int R>
@@ -363,24 +371,27 @@ cudaError_t dispatch(int mode, const CUtensorMap& mc, const CUtensorMap& mo, con
 
 bool step3d_available() { return true; }
 
-int plan_zchunk3d(int nz, int ny, int nx, int nshot) {
-    const long long columns = (long long)((ny + T3_TY - 1) / T3_TY) * ((nx + T3_TX - 1) / T3_TX) * nshot;
-    int best = T3_ZCHUNK;
+void plan_columns3d(int nz, int ny, int nx, int nshot, int* tile_x, int* planes) {
     double least = 0;
-    for (int n = (nz + T3_ZCHUNK - 1) / T3_ZCHUNK; n <= nz; ++n) {
-        const int chunk = (nz + n - 1) / n;
-        const long long ctas = columns * ((nz + chunk - 1) / chunk), slots = 2 * 152;
-        if (n > (nz + T3_ZCHUNK - 1) / T3_ZCHUNK && (chunk < 4 || ctas > 65535)) break;
-        // a lone CTA of an SM takes about 0.7 of the time of two for a plane
-        const double waves = ctas <= slots / 2 ? 0.7 : ctas < 4 * slots ? double((ctas + slots - 1) / slots)
-                                                                      : double(ctas) / slots + 0.5;
-        const double t = waves * (chunk + 6.0);
-        if (least == 0 || t < least) {
-            least = t;
-            best = chunk;
+    for (const int tx : {T3_TX, T3_TX2}) {
+        const int ty = T3_CELLS / tx, n0 = (nz + T3_ZCHUNK - 1) / T3_ZCHUNK;
+        const long long tiles = (long long)((ny + ty - 1) / ty) * ((nx + tx - 1) / tx), columns = tiles * nshot;
+        for (int n = n0; n <= nz; ++n) {
+            const int chunk = (nz + n - 1) / n;
+            const long long ctas = columns * ((nz + chunk - 1) / chunk), slots = 2 * 152;
+            if (tx != T3_TX && tiles * ((nz + chunk - 1) / chunk) > 65535) break;  // (gridDim.y)
+            if (n > n0 && (chunk < 4 || ctas > 65535)) break;
+            // a lone CTA of an SM takes about 0.7 of the time of two for a plane
+            const double waves = ctas <= slots / 2 ? 0.7 : ctas < 4 * slots ? double((ctas + slots - 1) / slots)
+                                                                          : double(ctas) / slots + 0.5;
+            const double t = waves * (chunk + 6.0);
+            if (least == 0 || t < least) {
+                least = t;
+                *tile_x = tx;
+                *planes = chunk;
+            }
         }
     }
-    return best;
 }
 
 cudaError_t launch_step3d(int R, int mode, const CUtensorMap& mc, const CUtensorMap& mo,

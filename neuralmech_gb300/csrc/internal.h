@@ -201,6 +201,7 @@ bool plan_resident(int nz, int nx, int R, int nshot, ResMode mode, ResPlan* out)
 struct ResArgs {
     StepArgs a;               // geometry, weights, m, sponge, point lists, gradient sum (adjoint)
     const float *u_in, *x_in; // the state: u_n and u_{n-1} (or d_n), [nshot][cells]; null: 0
+    int x_is_diff;            // x_in holds d_n = u_n - u_{n-1} for a leapfrog launch
     float *u_out, *x_out;     // the state after the last step (null: not written)
     float* lap;               // L u of the level at step it: lap + it lap_stride, from step lap_from
     long long lap_stride;     //   on (forward: written when not null; adjoint: read, q L u summed)

@@ -198,7 +198,14 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
 #pragma unroll
     for (int r = 0; r < RB; ++r) {
         X[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (active && p.x_in && zb + r < a.nz && x_ok) X[r] = f4(p.x_in + so + (long long)(zb + r) * a.ld + x);
+        if (active && p.x_in && zb + r < a.nz && x_ok) {
+            const long long off = so + (long long)(zb + r) * a.ld + x;
+            X[r] = f4(p.x_in + off);
+            if (MODE == RES_LEAP && p.x_is_diff) {
+                const float4 u = f4(p.u_in + off);
+                X[r] = make_float4(u.x - X[r].x, u.y - X[r].y, u.z - X[r].z, u.w - X[r].w);
+            }
+        }
     }
     float4 G[ADJ ? RB : 1];
 #pragma unroll

@@ -980,13 +980,15 @@ int run_forward_res(const wfd_problem* p, const Geom& g, const Layout& L, const 
     int rc = run.clear(g.rf.mail_bytes);
     if (rc) return rc;
     // FP32 checkpoints are the state itself: a launch leaves it in the next segment's slot
-    // and the next launch, the recompute's too, starts from there. (Packed and unpacked by
-    // kernels of their own, 4 launches a segment: the gradient of 4 shots of 187 x 243
-    // with 22 segments 4.01 -> 3.66 ms, of 320 x 650 with 24 5.11 -> 4.69.)
-    const bool direct = p->ckpt_format == WFD_CKPT_FP32;
+    // and the next launch, the recompute's too, starts from there. BF16 ones are written
+    // beside the state and read by the recompute. (Packed and unpacked by kernels of their
+    // own, 4 launches a segment: the gradient of 4 shots of 187 x 243 with 22 segments 4.01
+    // -> 3.66 ms, of 320 x 650 with 24 5.11 -> 4.69; with BF16, 300 steps, 2.61 -> 2.35
+    // and 2.69 -> 2.41.)
+    const bool f32 = p->ckpt_format == WFD_CKPT_FP32, bf16 = p->ckpt_format == WFD_CKPT_BF16;
     auto slot_of = [&](int n) { return w.ckpt + (size_t)(n / g.K) * 2 * L.ckpt_field_bytes; };
     if (save && g.jstore > 0) {  // (the checkpoint of level 0)
-        if (direct) {
+        if (f32 || bf16) {
             WFD_CUDA(cudaMemsetAsync(slot_of(0), 0, 2 * L.ckpt_field_bytes, s));
         } else {
             WFD_CUDA(cudaMemsetAsync(w.P[0], 0, L.field_bytes, s));
@@ -1000,18 +1002,23 @@ int run_forward_res(const wfd_problem* p, const Geom& g, const Layout& L, const 
         const int n1 = std::min(p->nt, n + seg);
         float* level[2] = {w.P[n & 1], w.P[n1 & 1]};
         float* other[2] = {summed ? w.D : w.P[(n + 1) & 1], summed ? w.D : w.P[(n1 + 1) & 1]};
+        ResArgs q{};
         for (int e = 0; e < 2; ++e) {  // the segment's start and end
             const int k = e == 0 ? n : n1;
             if (!save || k >= g.k0_store) continue;
-            if (direct) {
-                other[e] = reinterpret_cast<float*>(slot_of(k));
-                level[e] = reinterpret_cast<float*>(slot_of(k) + L.ckpt_field_bytes);
+            unsigned char *slot_x = slot_of(k), *slot_u = slot_x + L.ckpt_field_bytes;
+            if (f32) {
+                other[e] = reinterpret_cast<float*>(slot_x);
+                level[e] = reinterpret_cast<float*>(slot_u);
+            } else if (bf16) {
+                if (e == 0) continue;
+                q.u_bf16 = reinterpret_cast<uint2*>(slot_u);
+                q.x_bf16 = reinterpret_cast<uint2*>(slot_x);
             } else if (e == 0) {
-                WFD_CUDA(launch_pack(other[0], slot_of(k), n_all, p->ckpt_format, s));
-                WFD_CUDA(launch_pack(level[0], slot_of(k) + L.ckpt_field_bytes, n_all, p->ckpt_format, s));
+                WFD_CUDA(launch_pack(other[0], slot_x, n_all, p->ckpt_format, s));
+                WFD_CUDA(launch_pack(level[0], slot_u, n_all, p->ckpt_format, s));
             }
         }
-        ResArgs q{};
         q.a = st.base(nullptr);
         if (p->nsrc > 0) {
             q.a.inj = w.src;
@@ -1072,7 +1079,7 @@ int run_backward_res(const wfd_problem* p, const Geom& g, const Layout& L, const
         if (j < g.jstore) {
             PhaseScope scope(PH_RECOMPUTE, s, cdiv(p->nshot, g.rf.shots));
             const unsigned char* ck = w.ckpt + (size_t)j * 2 * L.ckpt_field_bytes;
-            const bool direct = p->ckpt_format == WFD_CKPT_FP32;  // (see run_forward_res)
+            const bool direct = p->ckpt_format != WFD_CKPT_I16;  // (see run_forward_res)
             const float *u = reinterpret_cast<const float*>(ck + L.ckpt_field_bytes),
                         *old = reinterpret_cast<const float*>(ck);
             if (!direct) {
@@ -1096,6 +1103,7 @@ int run_backward_res(const wfd_problem* p, const Geom& g, const Layout& L, const
             q.u_in = u;
             q.x_in = old;
             q.x_is_diff = direct && summed;
+            q.in_bf16 = p->ckpt_format == WFD_CKPT_BF16;
             q.lap = w.slot(L, 1);
             q.lap_stride = slot;
             q.steps = k1 - k0;

@@ -174,12 +174,16 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
     owned[gt] = NONE;
     // ---- u_n with its halo, m, and the second level
     const long long so = (long long)s * a.shot_stride;
+    auto state = [&](const float* from, long long off) {  // 4 cells of u_in or x_in
+        if (MODE == RES_LEAP && p.in_bf16) return unpack_bf16x4(reinterpret_cast<const uint2*>(from)[off / 4]);
+        return f4(from + off);
+    };
     if (active) {
         for (int k = gt; k < (tz + 2 * R) * (W / 4); k += GT) {
             const int row = k / (W / 4), c = k - row * (W / 4);
             const int z = z0 - R + row, xx = x0 - 4 + 4 * c;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (p.u_in && z >= 0 && z < a.nz && xx >= 0 && xx < a.ld) v = f4(p.u_in + so + (long long)z * a.ld + xx);
+            if (p.u_in && z >= 0 && z < a.nz && xx >= 0 && xx < a.ld) v = state(p.u_in, so + (long long)z * a.ld + xx);
             *reinterpret_cast<float4*>(U + row * W + 4 * c) = v;
         }
     }
@@ -200,9 +204,9 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
         X[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (active && p.x_in && zb + r < a.nz && x_ok) {
             const long long off = so + (long long)(zb + r) * a.ld + x;
-            X[r] = f4(p.x_in + off);
+            X[r] = state(p.x_in, off);
             if (MODE == RES_LEAP && p.x_is_diff) {
-                const float4 u = f4(p.u_in + off);
+                const float4 u = state(p.u_in, off);
                 X[r] = make_float4(u.x - X[r].x, u.y - X[r].y, u.z - X[r].z, u.w - X[r].w);
             }
         }
@@ -514,6 +518,10 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
         const long long at = gr.so + (long long)z * a.ld + x;
         if (p.u_out) *reinterpret_cast<float4*>(p.u_out + at) = f4(U + (tr0 + r + R) * W + 4 + 4 * lane);
         if (p.x_out) *reinterpret_cast<float4*>(p.x_out + at) = X[r];
+        if (!ADJ && p.u_bf16) {
+            p.u_bf16[at / 4] = pack_bf16x4(f4(U + (tr0 + r + R) * W + 4 + 4 * lane));
+            p.x_bf16[at / 4] = pack_bf16x4(X[r]);
+        }
         if constexpr (ADJ) {
             if (z < R || z >= a.nz - R) continue;
             float* gp = a.grad + (long long)z * a.ld + x;

@@ -33,7 +33,7 @@ extern "C" {
 #define WFD_ERR_CUDA (-3)      /* a CUDA runtime / driver call failed */
 #define WFD_ERR_UNSTABLE (-4)  /* vmax * dt violates the CFL bound of the stencil */
 #define WFD_ERR_POSITION (-5)  /* a source or receiver outside the updated interior */
-#define WFD_ERR_TIMEOUT (-6)   /* a kernel gave up waiting for a TMA tile */
+#define WFD_ERR_TIMEOUT (-6)   /* a kernel gave up waiting for a TMA tile or a neighbouring tile's halo */
 #define WFD_ERR_STATE (-7)     /* wfd_backward without a preceding checkpointed forward */
 
 /* Checkpoint snapshot formats (bytes per cell). */
@@ -257,7 +257,7 @@ int wfd_forward_static(const wfd_problem* p, const float* vel, const float* spon
  * Status of wfd_forward_static on the current device: synchronises `stream`,
  * returns the first device-side error that calls of wfd_forward_static have
  * recorded in the static array since the last call of this function
- * (WFD_ERR_TIMEOUT for a TMA wait that gave up, WFD_ERR_POSITION for a source
+ * (WFD_ERR_TIMEOUT for a wait that gave up, WFD_ERR_POSITION for a source
  * or receiver outside the interior, whose samples are then not written) or 0,
  * and clears it: wfd_status for the static array. The array's device address
  * is cached per device at the first call of either entry point and belongs to
@@ -472,8 +472,8 @@ int wfd_temporal_step(const float* u0, const float* u1, float* v0, float* v1, fl
  * division per cell. Within FP32 rounding of the reference expression (1e-5
  * relative L2 over many launches), as the reference's own build with
  * --use_fast_math (2D_wave_cuda_temporal.py, COMPILER_OPTIONS) is, not value
- * for value. The window of each CTA lives in registers. Any M_padded >= M; no
- * alignment requirement. No counterpart beyond temporal_step itself.
+ * for value. A warp advances a strip of columns row by row, every step a few rows
+ * behind the one before it. Any M_padded >= M; no alignment requirement. No counterpart beyond temporal_step itself.
  */
 int wfd_temporal_step_fast(const float* u0, const float* u1, float* v0, float* v1, float wavespeed, float dt,
                            float dx, float dy, int N, int M, int M_padded, void* stream);

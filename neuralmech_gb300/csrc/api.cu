@@ -338,7 +338,7 @@ namespace {
 // is below the streaming kernels' time. A forward streams in about 4 us a step at least
 // and 2 us plus 0.4 M cells per us otherwise. Measured, us a step, streaming / resident:
 // forward 256^2 4.1 / 2.0, 1024^2 5.7 / 4.1, 2048^2 11.1 / 6.7, 24 shots of 401 x 1203
-// 34 / 20; gradient (recompute included) 4 shots of 187 x 243 11.7 / 8.2, 4 shots of
+// 34 / 20; gradient (recompute included) 4 shots of 187 x 243 11.7 / 7.3, 4 shots of
 // 1024^2 41.6 / 30.0, 8 shots 72 / 61, 16 shots 118 / 118, 32 shots 211 / 230 (streamed).
 bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
     if (p->ndim != 2 || p->field_format != WFD_FIELD_FP32 || p->lap_store != WFD_LAP_AUTO ||

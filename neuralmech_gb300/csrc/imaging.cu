@@ -85,6 +85,8 @@ __global__ void analytic_kernel(const float* __restrict__ x, const float* __rest
 }
 
 constexpr int TFM_THREADS = 128;
+// How a time becomes a sample index (see tfm_index).
+enum TfmIndex : int { TFM_LATE, TFM_EARLY, TFM_ANY };
 constexpr int TFM_PAIRS = 4;
 template <int N>
 struct Count {
@@ -111,12 +113,12 @@ __device__ int row_length(const float* xp, const float* yp, int P) {
 
 // Bound by the latency of the gathers (87% of their sectors hit L1) and the instructions of a
 // pair: so TFM_PAIRS pairs have their samples in flight at once, the sample index takes no
-// integer conversion and no test for a time before the first sample unless t0 < 0 (EARLY),
-// half of an SM's on-chip memory is left to L1 (see the launch), and where the list is a
+// integer conversion where t + 2^23 holds it, and no test for a time before the first sample
+// unless t0 < 0 (INDEX, see tfm_index), half of an SM's on-chip memory is left to L1 (see the launch), and where the list is a
 // grid's, a CTA takes a block of 16 x 8 pixels, whose samples of a trace lie closer together
 // than a row's. 32 elements, 1500 samples, 512^2 pixels: 340 -> 250 us a call (one pair at a
 // time, 128 pixels of a row, all of the memory to tau).
-template <bool EARLY>
+template <TfmIndex INDEX>
 __global__ void __launch_bounds__(TFM_THREADS)
     tfm_kernel(const float2* __restrict__ h, int E, const float* __restrict__ xe,
                const float* __restrict__ ye, int nt, float inv_dt, float t0, float inv_c,
@@ -159,15 +161,23 @@ __global__ void __launch_bounds__(TFM_THREADS)
 #pragma unroll
                 for (int i = 0; i < N; ++i) {
                     const float t = (te + tr[i * TFM_THREADS]) * inv_dt;
-                    in[i] = t < last;
-                    // int(t) and its float without conversions: t + 2^23 rounded down holds floor(t)
-                    // in its low bits (a time before the first sample truncates towards 0 instead)
-                    const float b = __fadd_rd(t, 8388608.f);
-                    int k = __float_as_int(b) - 0x4B000000;
-                    float kf = b - 8388608.f;
-                    if (EARLY && t < 0.f) {
+                    int k;
+                    float kf;
+                    if (INDEX == TFM_ANY) {
                         k = int(t);
                         kf = float(k);
+                        in[i] = k < nt - 1;
+                    } else {
+                        in[i] = t < last;
+                        // int(t) and its float without conversions: t + 2^23 rounded down holds floor(t)
+                        // in its low bits (a time before the first sample truncates towards 0 instead)
+                        const float b = __fadd_rd(t, 8388608.f);
+                        k = __float_as_int(b) - 0x4B000000;
+                        kf = b - 8388608.f;
+                        if (INDEX == TFM_EARLY && t < 0.f) {
+                            k = int(t);
+                            kf = float(k);
+                        }
                     }
                     w[i] = (t - kf) * scale;
                     const float2* hp = hr + (in[i] ? k : 0);
@@ -222,11 +232,23 @@ cudaError_t launch_analytic(const float* traces, long long ntr, int nt, const fl
     return cudaGetLastError();
 }
 
+// The bits of t + 2^23 count samples while t < 2^23 (from there on floats lie 2 apart and
+// more): so for traces of up to 2^23 samples, and times that are numbers, which they are
+// unless t0 is none, or 1 / dt is 0 or infinite. The rest takes int(t) (TFM_ANY), in which a
+// time that is no number reads sample 0 and leaves no image.
+static TfmIndex tfm_index(int nt, float inv_dt, float t0) {
+    if (nt > (1 << 23) || !(inv_dt > 0.f && inv_dt <= 3.402823466e38f)) return TFM_ANY;
+    return t0 >= 0.f ? TFM_LATE : t0 < 0.f ? TFM_EARLY : TFM_ANY;
+}
+
 cudaError_t launch_tfm(const float2* h, int E, const float* xe, const float* ye, int nt, float dt,
                        float t0, float c, const float* xp, const float* yp, int P, int reciprocity,
                        float* image, cudaStream_t s) {
     const size_t smem = (size_t)E * TFM_THREADS * sizeof(float);
-    const auto kernel = t0 >= 0.f ? tfm_kernel<false> : tfm_kernel<true>;
+    const TfmIndex index = tfm_index(nt, 1.f / dt, t0);
+    const auto kernel = index == TFM_LATE    ? tfm_kernel<TFM_LATE>
+                        : index == TFM_EARLY ? tfm_kernel<TFM_EARLY>
+                                             : tfm_kernel<TFM_ANY>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;

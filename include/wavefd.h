@@ -195,8 +195,10 @@ int wfd_forward_final(const wfd_problem* p, const float* vel, const float* spong
  * shots; 0 on the fixed ring) and, when grad_wavelet is not NULL,
  * grad_wavelet [nshot][nt][nsrc] = (dF/dwavelet)^T dtraces. Uses the checkpoints
  * of the preceding wfd_forward(save_checkpoints = 1) on the same workspace and
- * inputs (give both calls the same workspace_bytes), recomputing the forward
- * per segment; one backward per forward.
+ * inputs, recomputing the forward per segment; one backward per forward. Both
+ * calls want the same workspace_bytes, from which the kernels and their layout
+ * follow: without such a forward the gradients are NaN and wfd_status returns
+ * WFD_ERR_STATE.
  * Together with wfd_forward this is the reference solver's gradient,
  * cuwave `misfit_gradient(sim, sources, gamma, sensors, observed)` as used by
  * projects/18_fwi/2D_fwi.py:40, for a cotangent the caller chooses.
@@ -328,8 +330,8 @@ uint64_t wfd_batch_launches(const wfd_batch* batch);
 int wfd_batch_free(wfd_batch* batch);
 
 /* Synchronises `stream`, returns the first device-side error recorded in the
- * workspace since the last call (WFD_ERR_TIMEOUT, WFD_ERR_POSITION) or 0, and
- * clears it. */
+ * workspace since the last call (WFD_ERR_TIMEOUT, WFD_ERR_POSITION, WFD_ERR_STATE)
+ * or 0, and clears it. */
 int wfd_status(void* workspace, void* stream);
 
 /* FP64 sum of squares of n FP32 values, added into the device double *out

@@ -851,14 +851,28 @@ wfd_problem group_problem(const wfd_problem* p, int g0) {
     return q;
 }
 
+// What a checkpointed forward and its backward have to agree on, as a word of the
+// workspace: the layout and the tiles that its point lists are made for.
+unsigned route_code(const wfd_problem* p, const Geom& g, const Layout& L) {
+    const Geom a = adjoint_geom(p, g);
+    const unsigned long long parts[] = {L.total, g.res, (unsigned long long)g.sb, (unsigned long long)g.tile_z,
+                                        (unsigned long long)g.tile_x, (unsigned long long)a.tile_z,
+                                        (unsigned long long)a.tile_x, (unsigned long long)g.K,
+                                        (unsigned long long)p->nt};
+    unsigned long long h = 14695981039346656037ull;  // (FNV-1a, by words)
+    for (const unsigned long long v : parts) h = (h ^ v) * 1099511628211ull;
+    return unsigned(h >> 32) | 1u;  // (never 0)
+}
+
+// route: route_code of a checkpointed forward, else 0.
 int setup(const wfd_problem* p, const Geom& g, const Work& w, const float* vel,
-          const int32_t* src, const int32_t* rec, cudaStream_t s, bool clear_status = true) {
+          const int32_t* src, const int32_t* rec, cudaStream_t s, bool clear_status = true, unsigned route = 0) {
     if (clear_status) WFD_CUDA(cudaMemsetAsync(w.err, 0, sizeof(unsigned), s));  // fresh status word
     if (g.vd)  // vel is kappa: k = kappa dt^2 / dx^2, b = 1 / rho
         WFD_CUDA(launch_vd_params(vel, w.rho, w.m, w.b, g.nz, g.nx, g.ld,
                                   float((double)p->dt * p->dt / ((double)p->dx * p->dx)), s));
     else
-        WFD_CUDA(launch_vel_to_m(vel, w.m, g.nz, g.ny, g.nx, g.ld, p->dt / p->dx, s));
+        WFD_CUDA(launch_vel_to_m(vel, w.m, g.nz, g.ny, g.nx, g.ld, p->dt / p->dx, w.err + 1, route, s));
     WFD_CUDA(launch_build_lists(src, p->nshot, p->nsrc, g.nz, g.ny, g.nx, g.ld, g.R, g.tile_z,
                                 g.tile_y, g.tile_x, g.tiles_z, g.tiles_y, g.tiles_x, w.counts,
                                 const_cast<int*>(w.src.off), const_cast<int2*>(w.src.ent), w.err, s));
@@ -1864,7 +1878,8 @@ int wfd_forward(const wfd_problem* p, const float* vel, const float* sponge_z,
     for (int g0 = 0; g0 < p->nshot; g0 += G) {
         const wfd_problem q = group_problem(p, g0);
         const Geom g = group_geom(&q, gf);
-        if ((rc = setup(&q, g, w, vel, src + 3L * g0 * p->nsrc, rec + 3L * g0 * p->nrec, s, g0 == 0)))
+        if ((rc = setup(&q, g, w, vel, src + 3L * g0 * p->nsrc, rec + 3L * g0 * p->nrec, s, g0 == 0,
+                        save_checkpoints ? route_code(&q, g, L) : 0)))
             return rc;
         Stepper st{&q, g, s, w.err, w.m, sponge_z, p->ndim == 3 ? sponge_y : nullptr, sponge_x};
         if ((rc = st.init())) return rc;
@@ -1923,6 +1938,20 @@ int wfd_backward(const wfd_problem* p, const float* vel, const float* sponge_z,
     if ((rc = check_workspace(workspace, workspace_bytes, L.total))) return rc;
     const Work w = carve(workspace, L, true);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const long long keys = (long long)p->nshot * g.ntiles + 1, akeys = (long long)p->nshot * adjoint_geom(p, g).ntiles + 1;
+    RouteLists lists{};
+    auto list = [&](int k, const PointLists& l, long long n) {
+        lists.off[k] = const_cast<int*>(l.off);
+        lists.n[k] = l.off ? n : 0;
+    };
+    list(0, w.src, keys);
+    list(1, w.rec, keys);
+    list(2, w.src_e, keys);
+    if (w.own_alists) {
+        list(3, w.src_a, akeys);
+        list(4, w.rec_a, akeys);
+    }
+    WFD_CUDA(launch_check_route(w.err, w.err + 1, route_code(p, g, L), lists, w.m, g.cells, s));
     Stepper st{p, g, s, w.err, w.m, sponge_z, p->ndim == 3 ? sponge_y : nullptr, sponge_x};
     if ((rc = st.init())) return rc;
     return run_backward(p, g, L, w, st, wavelet, dtraces, grad_vel, grad_wavelet, vel);
@@ -1963,7 +1992,7 @@ int misfit_gradient_impl(const wfd_problem* p, const float* vel, const float* sp
         const int32_t* grec = rec + 3L * g0 * p->nrec;
         const float* gwav = wavelet + (long long)g0 * p->nt * p->nsrc;
         const long long toff = (long long)g0 * p->nt * p->nrec;
-        if ((rc = setup(&q, g, w, vel, gsrc, grec, s, g0 == 0))) return rc;
+        if ((rc = setup(&q, g, w, vel, gsrc, grec, s, g0 == 0, route_code(&q, g, L)))) return rc;
         Stepper st{&q, g, s, w.err, w.m, sponge_z, p->ndim == 3 ? sponge_y : nullptr, sponge_x};
         if ((rc = st.init())) return rc;
         float* d = traces ? traces + toff : w.res;
@@ -2119,6 +2148,9 @@ int wfd_status(void* workspace, void* stream) {
     if (h & DEV_ERR_TMA_TIMEOUT) return fail(WFD_ERR_TIMEOUT, "device: TMA wait timed out");
     if (h & DEV_ERR_BAD_POSITION)
         return fail(WFD_ERR_POSITION, "device: a source/receiver lies outside the interior");
+    if (h & DEV_ERR_ROUTE)
+        return fail(WFD_ERR_STATE, "device: no checkpointed forward of this problem and workspace_bytes precedes "
+                                   "the backward");
     return WFD_OK;
 }
 

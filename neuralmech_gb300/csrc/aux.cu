@@ -11,7 +11,8 @@ namespace wfd {
 namespace {
 
 __global__ void vel_to_m_kernel(const float* __restrict__ vel, float* __restrict__ m, int nz,
-                                int ny, int nx, int ld, float scale) {
+                                int ny, int nx, int ld, float scale, unsigned* route, unsigned code) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *route = code;
     const long long n = (long long)nz * ny * ld;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
@@ -21,6 +22,19 @@ __global__ void vel_to_m_kernel(const float* __restrict__ vel, float* __restrict
         if (x < nx) v = vel[zy * nx + x] * scale;
         m[i] = v * v;
     }
+}
+
+// A backward on a workspace that a forward of another route (or none) has left: its lists
+// and fields lie elsewhere. Records it, empties the lists (whatever they hold is no index)
+// and leaves a model that makes the gradient NaN.
+__global__ void check_route_kernel(unsigned* err, const unsigned* route, unsigned code, RouteLists lists,
+                                   float* m, long long cells) {
+    if (*route == code) return;
+    const long long i0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    if (i0 == 0) report(err, DEV_ERR_ROUTE);
+    for (int k = 0; k < RouteLists::N; ++k)
+        for (long long i = i0; i < lists.n[k]; i += step) lists.off[k][i] = 0;
+    for (long long i = i0; i < cells; i += step) m[i] = __int_as_float(0x7fffffff);
 }
 
 __device__ __forceinline__ bool decode(const int32_t* pos, int nz, int ny, int nx, int R, int& z,
@@ -242,8 +256,15 @@ int grid_for(long long n, int block = 256) {
 }  // namespace
 
 cudaError_t launch_vel_to_m(const float* vel, float* m, int nz, int ny, int nx, int ld,
-                            float scale, cudaStream_t s) {
-    vel_to_m_kernel<<<grid_for((long long)nz * ny * ld), 256, 0, s>>>(vel, m, nz, ny, nx, ld, scale);
+                            float scale, unsigned* route, unsigned code, cudaStream_t s) {
+    vel_to_m_kernel<<<grid_for((long long)nz * ny * ld), 256, 0, s>>>(vel, m, nz, ny, nx, ld, scale, route, code);
+    count_launch();
+    return cudaGetLastError();
+}
+
+cudaError_t launch_check_route(unsigned* err, const unsigned* route, unsigned code, const RouteLists& lists,
+                               float* m, long long cells, cudaStream_t s) {
+    check_route_kernel<<<152, 256, 0, s>>>(err, route, code, lists, m, cells);
     count_launch();
     return cudaGetLastError();
 }

@@ -10,6 +10,7 @@ namespace wfd {
 enum : unsigned {
     DEV_ERR_TMA_TIMEOUT = 1u << 0,   // a wait for a TMA tile or a neighbour's halo gave up
     DEV_ERR_BAD_POSITION = 1u << 1,  // a source/receiver outside the updated interior
+    DEV_ERR_ROUTE = 1u << 2,         // a backward without a forward of its own layout
 };
 
 // ---------------------------------------------------------------- 2D tiles
@@ -326,8 +327,21 @@ int set_error(int status, const char* message);
 int auto_spc(int ntiles, int nshot, double share);
 
 // ---------------------------------------------------------------- helpers (aux.cu)
+// m = (vel scale)^2 on rows of ld cells; also leaves `code` in *route: which layout a
+// checkpointed forward gives the workspace (0: none).
 cudaError_t launch_vel_to_m(const float* vel, float* m, int nz, int ny, int nx, int ld,
-                            float scale, cudaStream_t s);
+                            float scale, unsigned* route, unsigned code, cudaStream_t s);
+// The offset arrays of a workspace's point lists.
+struct RouteLists {
+    static constexpr int N = 5;
+    int* off[N];
+    long long n[N];
+};
+// Nothing where *route is code; else DEV_ERR_ROUTE, no points and m = NaN. (One launch a
+// backward, which the host cannot spare: it knows the workspace's contents no more than
+// its caller does.)
+cudaError_t launch_check_route(unsigned* err, const unsigned* route, unsigned code, const RouteLists& lists,
+                               float* m, long long cells, cudaStream_t s);
 // Per-(shot, tile) point lists. With halo_z / halo_x > 0 a point joins every
 // tile whose region grown by that halo contains it (at most 4 in 2D); ent must
 // then hold 4 entries per point.

@@ -972,6 +972,9 @@ struct Resident {
             q.nshots = std::min(plan.shots, p->nshot - s0);
             q.tag0 = tag;
             tag += unsigned(q.steps);
+            // (a launch of one step: no tile waits for a neighbour between that one's load of
+            // its halo and its own stores. The leapfrog's old level is then u_in as it stands.)
+            if (q.steps == 1 && q.x_out == q.u_in) q.x_out = nullptr;
             const cudaError_t e = launch_resident(R, mode, plan, q, s);
             if (e != cudaSuccess) return fail(WFD_ERR_CUDA, "resident launch failed: %s", cudaGetErrorString(e));
         }

@@ -203,7 +203,8 @@ struct ResArgs {
     StepArgs a;               // geometry, weights, m, sponge, point lists, gradient sum (adjoint)
     const float *u_in, *x_in; // the state: u_n and u_{n-1} (or d_n), [nshot][cells]; null: 0
     int x_is_diff, in_bf16;   // leapfrog: x_in holds d_n = u_n - u_{n-1}; u_in and x_in are BF16
-    float *u_out, *x_out;     // the state after the last step (null: not written)
+    float *u_out, *x_out;     // the state after the last step (null: not written); with two
+                              // steps and more they may be u_in and x_in, with one not u_in
     uint2 *u_bf16, *x_bf16;   // ... and in BF16 (null: not written; both or neither)
     float* lap;               // L u of the level at step it: lap + it lap_stride, from step lap_from
     long long lap_stride;     //   on (forward: written when not null; adjoint: read, q L u summed)

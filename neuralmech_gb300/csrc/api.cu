@@ -106,23 +106,27 @@ using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, 
                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+// A driver function of CUDA 12.0 (null: not there).
+template <class F>
+F driver_entry(const char* name) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const bool ok = cudaGetDriverEntryPointByVersion(name, &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<F>(p) : nullptr;
+}
+
 EncodeTiled encoder() {
-    // cuTensorMapEncodeTiled wants a current context, and a thread that has made no
-    // runtime call yet (autograd's, on a first backward) has none
-    thread_local bool bound = false;
-    if (!bound) {
+    // cuTensorMapEncodeTiled wants a current context. A thread that has made no runtime call
+    // yet (autograd's, on a first backward) has none and gets its device's primary one; a
+    // context that the caller has made current stays.
+    static const auto get_current = driver_entry<CUresult (*)(CUcontext*)>("cuCtxGetCurrent");
+    CUcontext current = nullptr;
+    if (!get_current || get_current(&current) != CUDA_SUCCESS || !current) {
         int dev = 0;
-        bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaSetDevice(dev);
     }
-    static EncodeTiled fn = nullptr;
-    if (!fn) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                             cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiled>(p);
-    }
+    static const auto fn = driver_entry<EncodeTiled>("cuTensorMapEncodeTiled");
     return fn;
 }
 

@@ -230,9 +230,15 @@ def _require_cuda(t: torch.Tensor, name: str):
         raise ValueError(f"{name} must be a CUDA tensor (no CPU path)")
 
 
+def _as_positions(pos):
+    """An array or a tensor, where it lies, of positions in any form that torch.as_tensor
+    takes (lists, of device scalars too; device arrays of other libraries)."""
+    return pos if isinstance(pos, (np.ndarray, torch.Tensor)) else torch.as_tensor(pos)
+
+
 def _host_positions(pos, nshot: int, ndim: int) -> np.ndarray:
-    """_positions of positions that are on the host, there."""
-    p = np.asarray(pos)
+    """_positions of an array or a tensor that is on the host, there."""
+    p = pos.detach().to(torch.int32).numpy() if isinstance(pos, torch.Tensor) else pos
     if p.ndim == 2:
         p = np.broadcast_to(p, (nshot,) + p.shape)
     if p.ndim != 3 or p.shape[0] != nshot or p.shape[2] != ndim:
@@ -302,9 +308,9 @@ def _prepare(vel, wavelet, src, rec, grid: Grid, nshot=None) -> _Call:
         raise ValueError(f"vel has shape {tuple(vel.shape)}, grid {grid.shape}")
     vel = vel.detach().to(torch.float32).contiguous()
     dev = vel.device
+    src, rec = _as_positions(src), _as_positions(rec)
     if nshot is None:
-        shape = np.shape(src)
-        nshot = shape[0] if len(shape) == 3 else 1
+        nshot = src.shape[0] if src.ndim == 3 else 1
     # positions on the host travel with the sponge factors, in one copy
     on_host = [not (isinstance(p, torch.Tensor) and p.is_cuda) for p in (src, rec)]
     sp = sponge_profiles(grid)

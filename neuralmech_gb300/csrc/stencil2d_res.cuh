@@ -103,7 +103,8 @@ struct Weights {
 // What a group looks up in shared memory instead of keeping it in registers across steps.
 struct Group {
     long long so;            // offset of the shot in a field
-    int ilo, nlink, ihi;     // its tile's injected points: ent[ilo .. ihi), the first nlink linked
+    int ilo, nlink, ihi;     // its tile's injected points: ent[ilo .. ihi), linked (nlink of them) or
+                             // too many for that (nlink = -1)
     int slo, shi;            // its tile's sampled points
     int pad;
 };
@@ -119,7 +120,35 @@ struct Points {
 // (behind it, per thread of the group: its first point)
 constexpr unsigned NONE = 0xffffu;
 
-template <int R, int MODE, int RB>
+// A point's step value: g scale w (times m for a residual).
+__device__ __forceinline__ float point_value(const StepArgs& a, int cell, float w) {
+    float v = w * a.inj_scale;
+    if (a.inj_times_m) v *= __ldg(a.m + cell);
+    const int z = cell / a.ld, xx = cell - z * a.ld;
+    const float g = (a.gz ? __ldg(a.gz + z) : 1.f) * (a.gx ? __ldg(a.gx + xx) : 1.f);
+    return __fmul_rn(g, v);
+}
+
+// Injection into a tile that holds more points than are linked: all of them over all threads
+// of the group, by shared-memory atomics. (A thread that walked the list past the linked
+// points for its own cells: the gradient of 60 steps on 256^2 with a receiver in every cell
+// 6486 us, on 1024^2 16421; this way 1206 and 2566 (streaming kernels 1856 and 3070).)
+__device__ __forceinline__ void add_points(const StepArgs& a, const Group& gr, float* U, int z0, int x0, int R,
+                                           const float* ival, int grp, int gt, int GT) {
+    bar_group(grp, GT);
+#pragma unroll 2
+    for (int j = gr.ilo + gt; j < gr.ihi; j += GT) {
+        const int2 en = __ldg(a.inj.ent + j);
+        const int z = en.x / a.ld, xx = en.x - z * a.ld;
+        atomicAdd(U + (z - z0 + R) * W + (xx - x0 + 4), point_value(a, en.x, __ldg(ival + en.y)));
+    }
+    bar_group(grp, GT);
+}
+
+// MANY: a shot has more points to inject than a tile links (RES_PTS), so a tile may. (An
+// instance of its own: in the one kernel add_points cost the others' steps 1 to 7%, by
+// registers and by its place in the loop; without it they are 1% faster than with the walk.)
+template <int R, int MODE, int RB, bool MANY>
 __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __grid_constant__ ResArgs p) {
     constexpr bool ADJ = MODE == RES_ADJOINT;
     constexpr bool SUM = MODE == RES_SUMMED || MODE == RES_SUMMED_DIFF;
@@ -234,7 +263,7 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
         gr.ihi = active && a.inj.off ? a.inj.off[key + 1] : 0;
         gr.slo = active && a.smp.off ? a.smp.off[key] : 0;
         gr.shi = active && a.smp.off ? a.smp.off[key + 1] : 0;
-        gr.nlink = min(gr.ihi - gr.ilo, RES_PTS);
+        gr.nlink = !MANY || gr.ihi - gr.ilo <= RES_PTS ? gr.ihi - gr.ilo : -1;
     }
     __syncthreads();
     auto owner_at = [&](int cell, int& own, int& at) {  // the owning thread of a cell of the tile
@@ -263,14 +292,6 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
     __syncthreads();
     if (!active) return;
     const int nlink = gr.nlink, nsmp = gr.shi - gr.slo;
-    // a point's step value: g scale w (times m for a residual)
-    auto weight = [&](int cell, float w) {
-        float v = w * a.inj_scale;
-        if (a.inj_times_m) v *= __ldg(a.m + cell);
-        const int z = cell / a.ld, xx = cell - z * a.ld;
-        const float g = (a.gz ? __ldg(a.gz + z) : 1.f) * (a.gx ? __ldg(a.gx + xx) : 1.f);
-        return __fmul_rn(g, v);
-    };
     // ---- mailboxes: [tile item][parity][2 R rows x 64 + 4 tz packets]
     const int per = 2 * R * 64 + 4 * tz;
     const bool nb_n = tzi > 0, nb_s = tzi + 1 < a.tiles_z, nb_w = tx > 0, nb_e = tx + 1 < a.tiles_x;
@@ -347,8 +368,8 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
             }
         }
         // the step's injected values
-        if (gt < nlink) pt.v[gt] = weight(pt.cell[gt], iv);
-        for (int j = gt + GT; j < nlink; j += GT) pt.v[j] = weight(pt.cell[j], __ldg(ival + pt.p[j]));
+        if (gt < nlink) pt.v[gt] = point_value(a, pt.cell[gt], iv);
+        for (int j = gt + GT; j < nlink; j += GT) pt.v[j] = point_value(a, pt.cell[j], __ldg(ival + pt.p[j]));
 
         // ------------------------------------------------ the update, into X
         float* lap = p.lap && it >= p.lap_from ? p.lap + gr.so + (long long)it * p.lap_stride : nullptr;
@@ -473,11 +494,20 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
                 }
             };
             for (unsigned k = owned[gt]; k != NONE; k = pt.next[k]) add(pt.at[k], pt.v[k]);
-            for (int j = gr.ilo + RES_PTS; j < gr.ihi; ++j) {
-                const int2 en = a.inj.ent[j];
-                int owner, at;
-                owner_at(en.x, owner, at);
-                if (owner == gt) add(at, weight(en.x, __ldg(ival + en.y)));
+        }
+        if (MANY && nlink < 0) {
+#pragma unroll 1
+            for (int k = 0; k < (SUM ? 2 : 1); ++k) {  // u and, in the summed form, d in its place in U
+                add_points(a, gr, U, z0, x0, R, ival, grp, gt, GT);
+                if constexpr (SUM) {
+#pragma unroll
+                    for (int r = 0; r < RB; ++r) {
+                        float* cell = U + (row0 + r + R) * W + 4 + 4 * lane;
+                        const float4 c = f4(cell);
+                        *reinterpret_cast<float4*>(cell) = X[r];
+                        X[r] = c;
+                    }
+                }
             }
         }
         // ------------------------------------------------ and to the neighbours, from this warp's rows
@@ -536,7 +566,7 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
     }
 }
 
-template <int R, int MODE, int RB>
+template <int R, int MODE, int RB, bool MANY>
 cudaError_t launch_one(const ResArgs& q, size_t smem, int ctas, cudaStream_t s) {
     static std::atomic<unsigned long long> configured{0};  // bit d: done on device d
     int dev = 0;
@@ -544,7 +574,7 @@ cudaError_t launch_one(const ResArgs& q, size_t smem, int ctas, cudaStream_t s) 
     if (e != cudaSuccess) return e;
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_relaxed) & bit)) {
-        e = cudaFuncSetAttribute(res_kernel<R, MODE, RB>, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM);
+        e = cudaFuncSetAttribute(res_kernel<R, MODE, RB, MANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, RES_SMEM);
         if (e != cudaSuccess) return e;
         configured.fetch_or(bit, std::memory_order_relaxed);
     }
@@ -558,26 +588,32 @@ cudaError_t launch_one(const ResArgs& q, size_t smem, int ctas, cudaStream_t s) 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, res_kernel<R, MODE, RB>, q);
+    e = cudaLaunchKernelEx(&cfg, res_kernel<R, MODE, RB, MANY>, q);
     count_launch();
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-template <int R, int MODE>
-cudaError_t launch_rb(int rb, const ResArgs& q, size_t smem, int ctas, cudaStream_t s) {
+template <int R, int MODE, bool MANY>
+cudaError_t launch_points(int rb, const ResArgs& q, size_t smem, int ctas, cudaStream_t s) {
     switch (rb) {
-        case 2: return launch_one<R, MODE, 2>(q, smem, ctas, s);
-        case 4: return launch_one<R, MODE, 4>(q, smem, ctas, s);
-        case 7: return launch_one<R, MODE, 7>(q, smem, ctas, s);
+        case 2: return launch_one<R, MODE, 2, MANY>(q, smem, ctas, s);
+        case 4: return launch_one<R, MODE, 4, MANY>(q, smem, ctas, s);
+        case 7: return launch_one<R, MODE, 7, MANY>(q, smem, ctas, s);
         case 10:
-            if constexpr (MODE != RES_ADJOINT) return launch_one<R, MODE, 10>(q, smem, ctas, s);
+            if constexpr (MODE != RES_ADJOINT) return launch_one<R, MODE, 10, MANY>(q, smem, ctas, s);
             return cudaErrorInvalidValue;
-        case 14: return launch_one<R, MODE, 14>(q, smem, ctas, s);
+        case 14: return launch_one<R, MODE, 14, MANY>(q, smem, ctas, s);
         case 19:
-            if constexpr (MODE != RES_ADJOINT) return launch_one<R, MODE, 19>(q, smem, ctas, s);
+            if constexpr (MODE != RES_ADJOINT) return launch_one<R, MODE, 19, MANY>(q, smem, ctas, s);
             return cudaErrorInvalidValue;
         default: return cudaErrorInvalidValue;
     }
+}
+
+template <int R, int MODE>
+cudaError_t launch_rb(int rb, const ResArgs& q, size_t smem, int ctas, cudaStream_t s) {
+    return q.a.inj_np > RES_PTS ? launch_points<R, MODE, true>(rb, q, smem, ctas, s)
+                                : launch_points<R, MODE, false>(rb, q, smem, ctas, s);
 }
 
 }  // namespace res

@@ -24,6 +24,7 @@ from __future__ import annotations
 
 import ctypes
 import dataclasses
+import math
 
 import torch
 
@@ -47,6 +48,37 @@ def _level_shares(models, budget: float) -> list:
         want.append(4.0 * cells * m["observed"].shape[0] * (g.nt + 1))
     total = sum(want)
     return [min(w, budget * w / total) for w in want]
+
+
+def _auto_spc(ntiles: int, nshot: int, share: float) -> int:
+    """Shots per CTA of a streaming kernel whose work runs `share` times side by side: the
+    library's rule (auto_spc in csrc/api.cu, which has the measurements)."""
+    best, least = 1, 0.0
+    for s in range(1, min(nshot, 64) + 1):
+        groups = -(-nshot // s)
+        if groups > 65535:
+            continue
+        t = max(share * ntiles * (nshot + 0.55 * groups) / 304.0, s + 0.55) + 0.45 * (s + 0.55)
+        if least == 0 or t < least:
+            best, least = s, t
+    return best
+
+
+def _batch_grids(grids, nshots) -> list:
+    """The grids of models that run side by side. 2D models without a tiling of their own
+    get the shots per CTA that wfd_batch_plan gives them, from the whole batch's work: it
+    asks for the streaming kernels, which share the chip (the resident one wants all of it
+    for a segment of steps), and holds for the graph as for the eager calls."""
+    if len(grids) < 2:
+        return list(grids)
+    cells = [float(math.prod((g.shape[0], g.shape[-1]))) for g in grids]
+    work = sum(n * c for n, c in zip(nshots, cells))
+    out = []
+    for g, n, c in zip(grids, nshots, cells):
+        if g.ndim == 2 and g.shots_per_cta == 0 and g.tile_rows == 0 and g.step_block <= 2:
+            g = dataclasses.replace(g, shots_per_cta=_auto_spc(max(1, int(c / 3000)), n, work / (c * n)))
+        out.append(g)
+    return out
 
 
 @dataclasses.dataclass
@@ -81,12 +113,13 @@ class BatchFWI:
         self.device = models[0]["vel"].device
         self.models = []
         shares = _level_shares(models, level_budget)
-        for m, share in zip(models, shares):
-            grid: Grid = m["grid"]
+        nshots = [m["observed"].shape[0] for m in models]
+        grids = [m["grid"] for m in models]
+        if autotune:
+            grids = [_autotune.tuned(g, n, vel=m["vel"], for_gradient=True, **(tune_kw or {}))
+                     for g, n, m in zip(grids, nshots, models)]
+        for m, share, nshot, grid in zip(models, shares, nshots, _batch_grids(grids, nshots)):
             obs = m["observed"].to(torch.float32).contiguous()
-            nshot = obs.shape[0]
-            if autotune:
-                grid = _autotune.tuned(grid, nshot, vel=m["vel"], for_gradient=True, **(tune_kw or {}))
             if share > 0:
                 grid = dataclasses.replace(grid, store_levels=levels_for_budget(grid, nshot, share))
             call = _prepare(m["vel"], torch.as_tensor(m["wavelet"], device=self.device), m["src"], m["rec"],
@@ -100,10 +133,6 @@ class BatchFWI:
         self.graph = None  # the library's batch plan (its graph), when graph=True
         self.graph_kernels = 0  # kernels of one replay
         if not graph:
-            for m in self.models:  # side by side: the streaming kernels, as the library's plan does
-                p = m.call.problem
-                if len(self.models) > 1 and p.ndim == 2 and p.tile_rows == 0 and p.shots_per_cta == 0:
-                    p.tile_rows = 32
             self._launch()  # eager run: validates arguments
             torch.cuda.synchronize(self.device)
             return

@@ -96,8 +96,8 @@ class BatchFWI:
 
     models: sequence of dicts with keys vel (nz, nx) CUDA tensor, wavelet,
     src, rec (as for ``wave_forward``), observed (nshot, nt, nrec) CUDA tensor
-    and grid (``Grid``). ``autotune`` picks tile_rows / shots_per_cta per
-    model; ``graph=False`` runs the same calls eagerly on the streams.
+    and grid (``Grid``). ``autotune`` picks the steps per launch of each model (of a
+    batch of one, the whole configuration); ``graph=False`` runs the same calls eagerly on the streams.
     ``level_budget`` (bytes) is shared among the models' adjoints for the
     forward levels they keep instead of recomputing (``Grid.store_levels``),
     in proportion to the levels each would keep with unlimited memory (a
@@ -116,7 +116,8 @@ class BatchFWI:
         nshots = [m["observed"].shape[0] for m in models]
         grids = [m["grid"] for m in models]
         if autotune:
-            grids = [_autotune.tuned(g, n, vel=m["vel"], for_gradient=True, **(tune_kw or {}))
+            grids = [_autotune.tuned(g, n, vel=m["vel"], for_gradient=True, batch=len(models) > 1,
+                                     **(tune_kw or {}))
                      for g, n, m in zip(grids, nshots, models)]
         for m, share, nshot, grid in zip(models, shares, nshots, _batch_grids(grids, nshots)):
             obs = m["observed"].to(torch.float32).contiguous()

@@ -85,6 +85,7 @@ __global__ void analytic_kernel(const float* __restrict__ x, const float* __rest
 }
 
 constexpr int TFM_THREADS = 128;
+constexpr int TFM_MAX_ELEMENTS = 256;  // (wfd_tfm checks)
 // How a time becomes a sample index (see tfm_index).
 enum TfmIndex : int { TFM_LATE, TFM_EARLY, TFM_ANY };
 constexpr int TFM_PAIRS = 4;
@@ -253,10 +254,11 @@ cudaError_t launch_tfm(const float2* h, int E, const float* xe, const float* ye,
     const auto kernel = index == TFM_LATE    ? tfm_kernel<TFM_LATE>
                         : index == TFM_EARLY ? tfm_kernel<TFM_EARLY>
                                              : tfm_kernel<TFM_ANY>;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    // (the limit for the most elements, whatever this call has: with row_length's two words
+    // 48 KB of tau, 96 elements, are past the default one too)
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               int(TFM_MAX_ELEMENTS * TFM_THREADS * sizeof(float)));
+    if (e != cudaSuccess) return e;
     // (the gathers need L1 more than they need the last CTAs: 250 against 283 us at 38%, 273 at 75%)
     const cudaError_t pref = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
     if (pref != cudaSuccess) return pref;

@@ -21,6 +21,7 @@
 // the read-only path; they are L2-resident for the array sizes of the
 // reference drivers.
 #include <algorithm>
+#include <atomic>
 
 #include "common.cuh"
 #include "internal.h"
@@ -246,6 +247,14 @@ static TfmIndex tfm_index(int nt, float inv_dt, float t0) {
     return t0 >= 0.f ? TFM_LATE : t0 < 0.f ? TFM_EARLY : TFM_ANY;
 }
 
+// Share of an SM's on-chip memory for tau. The gathers need L1 more than they need the last
+// CTAs, so half, unless that leaves only three CTAs where a little more gives four, or one where
+// all of it gives two. us a call, half / the share taken, pixels of a grid (scattered ones):
+// 64 elements, 65536 pixels 526 / 329 (772 / 515); 56, 262144 776 / 627 (1387 / 1260); 200, 65536
+// 8384 / 4325 (17198 / 8982). 32, 262144 with half / three quarters 242 / 242 (546 / 654); 96, 262144
+// with half / all 3430 / 1998 (4206 / 6692).
+static int tfm_carveout(int E) { return E > 128 ? 100 : E > 48 && E <= 64 ? 60 : 50; }
+
 cudaError_t launch_tfm(const float2* h, int E, const float* xe, const float* ye, int nt, float dt,
                        float t0, float c, const float* xp, const float* yp, int P, int reciprocity,
                        float* image, cudaStream_t s) {
@@ -254,14 +263,22 @@ cudaError_t launch_tfm(const float2* h, int E, const float* xe, const float* ye,
     const auto kernel = index == TFM_LATE    ? tfm_kernel<TFM_LATE>
                         : index == TFM_EARLY ? tfm_kernel<TFM_EARLY>
                                              : tfm_kernel<TFM_ANY>;
-    // (the limit for the most elements, whatever this call has: with row_length's two words
-    // 48 KB of tau, 96 elements, are past the default one too)
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               int(TFM_MAX_ELEMENTS * TFM_THREADS * sizeof(float)));
+    // What the launch wants of the kernel; asked for when it is another than the last launch's
+    // on the device (two calls of the runtime are 5% of a small image's). The limit of shared
+    // memory is the one for the most elements, whatever this call has: with row_length's two
+    // words 48 KB of tau, 96 elements, are past the default one too.
+    static std::atomic<int> set[3][64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    // (the gathers need L1 more than they need the last CTAs: 250 against 283 us at 38%, 273 at 75%)
-    const cudaError_t pref = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 50);
-    if (pref != cudaSuccess) return pref;
+    const int carveout = tfm_carveout(E);
+    if (set[index][dev & 63].load(std::memory_order_relaxed) != carveout) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(TFM_MAX_ELEMENTS * TFM_THREADS * sizeof(float)));
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+        if (e != cudaSuccess) return e;
+        set[index][dev & 63].store(carveout, std::memory_order_relaxed);
+    }
     // (blocks at the edges of a grid of pixels are partly empty: a CTA takes another one)
     kernel<<<(P + TFM_THREADS - 1) / TFM_THREADS, TFM_THREADS, smem, s>>>(
         h, E, xe, ye, nt, 1.f / dt, t0, 1.f / c, xp, yp, P, reciprocity, image);

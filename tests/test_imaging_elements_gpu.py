@@ -22,3 +22,26 @@ def test_tfm_element_counts(cuda, E):
     ref = tfm_kernel_semantics(h.astype(np.complex128), el[:, 0].astype(np.float64), el[:, 1].astype(np.float64), 0.01, 0.04,
                                1.0, x, y)
     assert rel_l2(img.cpu().numpy().ravel(), ref) < 1e-4
+
+
+def test_scattered_pixels_of_64_elements_are_not_slow(cuda):
+    """A pair of 64 elements costs no more than one of 48 (0.87 of it; with room for three CTAs
+    on an SM instead of four, 1.30)."""
+    from neuralmech_gb300.imaging import tfm
+
+    def us_a_pair(E):
+        gen = torch.Generator(device=cuda).manual_seed(E)
+        h = torch.view_as_complex(torch.randn((E, E, 1000, 2), generator=gen, device=cuda))
+        el = torch.stack([torch.linspace(0, 1, E), torch.zeros(E)], 1)
+        x, y = (torch.rand(65536, generator=gen, device=cuda) for _ in range(2))
+        best = float("inf")
+        for _ in range(6):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            tfm(h, el, 0.0, 0.0025, 1.0, x, y)
+            e[1].record()
+            torch.cuda.synchronize()
+            best = min(best, e[0].elapsed_time(e[1]))
+        return best / (E * (E + 1) / 2)
+
+    assert us_a_pair(64) < 1.1 * us_a_pair(48)

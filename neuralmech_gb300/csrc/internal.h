@@ -170,7 +170,8 @@ constexpr int res_threads(int mode, int rb) {
 }
 // Rows of a warp whose m may come from L2 instead of shared memory (the largest tiles).
 constexpr int res_l2_rows(int rb) { return rb >= 19 ? 6 : 0; }
-constexpr int RES_PTS = 256;       // injected points linked per tile (a tile with more adds them from the list)
+constexpr int RES_PTS = 256;       // injected points linked per tile
+constexpr int RES_WALK = 64;       // ... and looked up in its list by every thread, at most
 constexpr int RES_SMS = 152;       // CTAs that are resident at once, one per SM
 constexpr int RES_SMEM = 227 * 1024;
 

@@ -103,8 +103,8 @@ struct Weights {
 // What a group looks up in shared memory instead of keeping it in registers across steps.
 struct Group {
     long long so;            // offset of the shot in a field
-    int ilo, nlink, ihi;     // its tile's injected points: ent[ilo .. ihi), linked (nlink of them) or
-                             // too many for that (nlink = -1)
+    int ilo, nlink, ihi;     // its tile's injected points: ent[ilo .. ihi), the first nlink linked
+                             // (-1: too many, add_points)
     int slo, shi;            // its tile's sampled points
     int pad;
 };
@@ -129,10 +129,10 @@ __device__ __forceinline__ float point_value(const StepArgs& a, int cell, float 
     return __fmul_rn(g, v);
 }
 
-// Injection into a tile that holds more points than are linked: all of them over all threads
-// of the group, by shared-memory atomics. (A thread that walked the list past the linked
+// Injection into a tile that holds many more points than are linked: all of them over all
+// threads of the group, by shared-memory atomics. (By a walk of every thread past the linked
 // points for its own cells: the gradient of 60 steps on 256^2 with a receiver in every cell
-// 6486 us, on 1024^2 16421; this way 1206 and 2566 (streaming kernels 1856 and 3070).)
+// 6486 us, on 1024^2 16421; this way 1206 and 2566, streaming kernels 1856 and 3070.)
 __device__ __forceinline__ void add_points(const StepArgs& a, const Group& gr, float* U, int z0, int x0, int R,
                                            const float* ival, int grp, int gt, int GT) {
     bar_group(grp, GT);
@@ -145,9 +145,10 @@ __device__ __forceinline__ void add_points(const StepArgs& a, const Group& gr, f
     bar_group(grp, GT);
 }
 
-// MANY: a shot has more points to inject than a tile links (RES_PTS), so a tile may. (An
-// instance of its own: in the one kernel add_points cost the others' steps 1 to 7%, by
-// registers and by its place in the loop; without it they are 1% faster than with the walk.)
+// MANY: a shot has so many points to inject that the walk past a tile's linked ones may be
+// long (RES_WALK). An instance of its own: in the one kernel add_points costs the others' steps
+// 1 to 7%, by registers and by its place in the loop (and without the walk in its place the
+// order-8 forward at 2048^2 is 2% slower too).
 template <int R, int MODE, int RB, bool MANY>
 __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __grid_constant__ ResArgs p) {
     constexpr bool ADJ = MODE == RES_ADJOINT;
@@ -263,7 +264,7 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
         gr.ihi = active && a.inj.off ? a.inj.off[key + 1] : 0;
         gr.slo = active && a.smp.off ? a.smp.off[key] : 0;
         gr.shi = active && a.smp.off ? a.smp.off[key + 1] : 0;
-        gr.nlink = !MANY || gr.ihi - gr.ilo <= RES_PTS ? gr.ihi - gr.ilo : -1;
+        gr.nlink = !MANY || gr.ihi - gr.ilo <= RES_PTS ? min(gr.ihi - gr.ilo, RES_PTS) : -1;
     }
     __syncthreads();
     auto owner_at = [&](int cell, int& own, int& at) {  // the owning thread of a cell of the tile
@@ -494,6 +495,12 @@ __global__ void __launch_bounds__(res_threads(MODE, RB), 1) res_kernel(const __g
                 }
             };
             for (unsigned k = owned[gt]; k != NONE; k = pt.next[k]) add(pt.at[k], pt.v[k]);
+            for (int j = gr.ilo + RES_PTS; !MANY && j < gr.ihi; ++j) {  // (at most RES_WALK)
+                const int2 en = a.inj.ent[j];
+                int owner, at;
+                owner_at(en.x, owner, at);
+                if (owner == gt) add(at, point_value(a, en.x, __ldg(ival + en.y)));
+            }
         }
         if (MANY && nlink < 0) {
 #pragma unroll 1
@@ -612,7 +619,7 @@ cudaError_t launch_points(int rb, const ResArgs& q, size_t smem, int ctas, cudaS
 
 template <int R, int MODE>
 cudaError_t launch_rb(int rb, const ResArgs& q, size_t smem, int ctas, cudaStream_t s) {
-    return q.a.inj_np > RES_PTS ? launch_points<R, MODE, true>(rb, q, smem, ctas, s)
+    return q.a.inj_np > RES_PTS + RES_WALK ? launch_points<R, MODE, true>(rb, q, smem, ctas, s)
                                 : launch_points<R, MODE, false>(rb, q, smem, ctas, s);
 }
 

@@ -453,9 +453,10 @@ cudaError_t launch_temporal_stream(const float* u0, const float* u1, float* v0, 
     const int strips = (M + TS_COLS - 1) / TS_COLS;
     // Rows per warp. A warp spends 16 rows on its first and last results. A row takes it
     // 0.33 us alone and 0.045 more for each warp of its SM, up to the 12 that are resident;
-    // beyond them, more and shorter strips even out the SMs. Measured with S folded into Q,
-    // us: 256^2 8 rows 14.3, 16 rows 18.4; 2048^2 32 rows 35, 20 rows 39, 64 rows 43;
-    // 8000 x 16000 167 rows 425, 250 rows 441, 471 rows 543, 1000 rows 676.
+    // beyond them, more and shorter strips even out the SMs. Measured, us (the rule's choice
+    // first): 256^2 4 rows 14.4, 8 rows 17.1, 32 rows 31.2; 1000^2 10 rows 23.6, 24 rows 27.1; 2048^2
+    // 26 rows 43.8, 32 rows 37.5, 64 rows 49.7; 4000^2 44 rows 95.6, 80 rows 91.6, 128 rows 107.3;
+    // 8000 x 16000 127 rows 463, 250 rows 484, 471 rows 589, 1000 rows 735.
     int rows = N;
     double least = 0;
     for (int q = 1; q <= 64; ++q) {

@@ -13,9 +13,12 @@ cudaError_t launch_resident_r4(ResMode, int, const ResArgs&, size_t, int, cudaSt
 namespace {
 // A split's time per step, in microseconds: a latency of 2.2 (halo packets through
 // L2: about 1; two barriers; the send) plus the rows of a warp times what one row
-// costs at n warps per scheduler. Fitted to the order-8 leapfrog forward on 256^2 ..
-// 2048^2 and 1 .. 40 shots, within 15%: rb 2, 4 warps 2.2 us; 14, 4 warps 3.7; 19, 12
-// warps 7.7; 7, 16 warps 5.8. The adjoint reads L u from HBM and sums the gradient.
+// costs at n warps per scheduler. It orders the splits by their rows and warps; as a time
+// it is high, most of all at orders 2 and 4, so that some grids stream which would be
+// faster resident, and none the other way round. us a step, estimate / measured, order 8
+// (order 2): 256^2 2.45 / 1.56 (1.27); 1024^2 3.6 / 2.6 (1.9); 2040^2 7.8 / 6.3 (5.5); 24 shots of 401 x 1203
+// 25.3 / 19.3 (14.2); 6 of 700^2 7.8 / 6.7 (5.7). The adjoint reads L u from HBM and sums
+// the gradient.
 double step_us(int rb, int warps, bool adjoint) {
     static const double row[5] = {0.0, 0.125, 0.2, 0.295, 0.5};
     const double t = rb * row[(warps + 3) / 4];

@@ -26,8 +26,9 @@
 // tile writes level n + 2 only after it has received its neighbour's level
 // n + 1, which the neighbour wrote after its CTA barrier behind the read of
 // level n. The launch is cooperative, so every tile is resident. Every wait is
-// bounded; one that gives up records DEV_ERR_TMA_TIMEOUT and the launch runs to
-// its end without further waiting.
+// bounded; one that gives up records DEV_ERR_TMA_TIMEOUT, and its CTA goes on
+// without further waiting, which overtakes its neighbours' tags: theirs give up in
+// turn, each CTA once, and the launch runs to its end.
 //
 // Arithmetic. The cell updates are those of the streaming kernels, operation
 // for operation (lap_row, lap_row_diff, the update with its sponge factors),

@@ -72,7 +72,9 @@ class Grid:
              kernel)
     step_block   2D time steps per kernel launch, 1 or 2 (0 = 1); for a
              forward (no gradient) with the leapfrog update and FP32 fields
-             also 8 at order 2 or 4 at order 4 (a register window per CTA)
+             also 8 at order 2 or 4 at order 4 (a register window per CTA;
+             on grids up to about 2048^2 slower than 0, which takes the
+             resident kernel there)
     store_levels levels the adjoint's workspace may hold (lap_store "auto"):
              the forward keeps the levels of its last (store_levels - 2) // K
              segments and only the earlier ones are recomputed (0: the last

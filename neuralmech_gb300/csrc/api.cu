@@ -341,8 +341,8 @@ namespace {
 // gradient also with the adjoint's gradient sum in registers), where its estimate
 // is below the streaming kernels' time. A forward streams in about 4 us a step at least
 // and 2 us plus 0.4 M cells per us otherwise. Measured, us a step, streaming / resident:
-// forward 256^2 4.1 / 2.0, 1024^2 5.7 / 4.1, 2048^2 11.1 / 6.7, 24 shots of 401 x 1203
-// 34 / 20; gradient (recompute included) 4 shots of 187 x 243 11.7 / 7.3, 4 shots of
+// forward 256^2 4.1 / 1.8, 1024^2 5.7 / 2.6, 2048^2 11.1 / 6.5, 24 shots of 401 x 1203
+// 34 / 19; gradient (recompute included) 4 shots of 187 x 243 11.7 / 7.3, 4 shots of
 // 1024^2 41.6 / 30.0, 8 shots 72 / 61, 16 shots 118 / 118, 32 shots 211 / 230 (streamed).
 bool resident_plan(const wfd_problem* p, bool grad, ResPlan* f, ResPlan* a) {
     if (p->ndim != 2 || p->field_format != WFD_FIELD_FP32 || p->lap_store != WFD_LAP_AUTO ||
@@ -428,6 +428,13 @@ Geom make_geom(const wfd_problem* p, int tile_rows = 0, int step_block = 0, bool
         g.spc = 1;  // a 3D CTA works on one shot
     } else if (p->shots_per_cta > 0) {
         g.spc = std::min(std::min(p->shots_per_cta, p->nshot), T2_MAX_SPC);
+    } else if (p->field_format == WFD_FIELD_I16) {
+        // Int16 fields spend their time on the levels' coding, not on a CTA's start: powers of two
+        // that leave six waves of CTAs, as auto_spc has not: 8 shots of 1024^2, 60 steps 2833 us
+        // against 2909, 48 of 300^2 2256 against 2312.
+        int s = 1;
+        while (2LL * s <= (long long)g.ntiles * p->nshot / (6 * 304) && 2 * s <= p->nshot) s *= 2;
+        g.spc = std::min(s, T2_MAX_SPC);
     } else {
         g.spc = auto_spc(g.ntiles, p->nshot, 1.0);
     }

@@ -96,7 +96,7 @@ class BatchFWI:
 
     models: sequence of dicts with keys vel (nz, nx) CUDA tensor, wavelet,
     src, rec (as for ``wave_forward``), observed (nshot, nt, nrec) CUDA tensor
-    and grid (``Grid``). ``autotune`` picks the steps per launch of each model (of a
+    and grid (``Grid``). ``autotune`` picks the steps per launch of the models (of a
     batch of one, the whole configuration); ``graph=False`` runs the same calls eagerly on the streams.
     ``level_budget`` (bytes) is shared among the models' adjoints for the
     forward levels they keep instead of recomputing (``Grid.store_levels``),
@@ -115,10 +115,12 @@ class BatchFWI:
         shares = _level_shares(models, level_budget)
         nshots = [m["observed"].shape[0] for m in models]
         grids = [m["grid"] for m in models]
-        if autotune:
-            grids = [_autotune.tuned(g, n, vel=m["vel"], for_gradient=True, batch=len(models) > 1,
-                                     **(tune_kw or {}))
-                     for g, n, m in zip(grids, nshots, models)]
+        if autotune and len(models) > 1:
+            plain = [dataclasses.replace(g, tile_rows=0, shots_per_cta=0, step_block=0) for g in grids]
+            spcs = [g.shots_per_cta for g in _batch_grids(plain, nshots)]
+            grids = _autotune.tune_batch(grids, nshots, spcs, vels=[m["vel"] for m in models], **(tune_kw or {}))
+        elif autotune:
+            grids = [_autotune.tuned(grids[0], nshots[0], vel=models[0]["vel"], for_gradient=True, **(tune_kw or {}))]
         for m, share, nshot, grid in zip(models, shares, nshots, _batch_grids(grids, nshots)):
             obs = m["observed"].to(torch.float32).contiguous()
             if share > 0:

@@ -271,7 +271,7 @@ def _to_device(arrays, device) -> list:
     for a in arrays:
         at.append(n)
         n += 0 if a is None else (a.nbytes + 255) // 256 * 256
-    host = np.empty(n, np.uint8)
+    host = np.empty(max(n, 1), np.uint8)  # (an empty tensor cannot be viewed as another type)
     for a, o in zip(arrays, at):
         if a is not None:
             host[o:o + a.nbytes] = a.reshape(-1).view(np.uint8)

@@ -52,3 +52,25 @@ def test_device_positions(cuda, form):
     c = _prepare(torch.full((40, 60), 1500.0, device=cuda), np.zeros(10), pos, CELLS, grid)
     assert c.src.device == c.rec.device == c.vel.device
     assert torch.equal(c.src, c.rec) and c.src[0, :, 0].tolist() == [20, 9, 12] and c.src[0, :, 2].tolist() == [31, 44, 12]
+
+
+@pytest.mark.parametrize("sponge", [0, 3])
+def test_no_points_at_all(sponge):
+    """Neither sources nor receivers, with and without a sponge: the one copy may hold nothing."""
+    from neuralmech_gb300.wavefd import Grid, _host_positions, _to_device, sponge_profiles
+    none = _host_positions(np.zeros((2, 0, 2), np.int32), 2, 2)
+    profiles = sponge_profiles(Grid((40, 60), (10.0, 10.0), 1e-3, 10, sponge=sponge))
+    src, rec, gz, gy, gx = _to_device([none, none, *profiles], "cpu")
+    assert src.shape == rec.shape == (2, 0, 3) and src.dtype == torch.int32 and gy is None
+    assert (gz is None and gx is None) if sponge == 0 else (gz.shape == (40,) and gx.shape == (60,))
+
+
+@pytest.mark.gpu
+def test_no_points_in_a_call(cuda):
+    from neuralmech_gb300.wavefd import Grid, misfit_gradient, wave_forward
+    grid = Grid((40, 60), (10.0, 10.0), 1e-3, 10, sponge=0)
+    vel = torch.full((40, 60), 1500.0, device=cuda)
+    none, wav = np.zeros((2, 0, 2), np.int32), torch.zeros((2, 10, 0), device=cuda)
+    assert wave_forward(vel, wav, none, none, grid).shape == (2, 10, 0)
+    J, g = misfit_gradient(vel, wav, none, none, torch.zeros((2, 10, 0), device=cuda), grid)
+    assert float(J) == 0 and not bool(g.any())
